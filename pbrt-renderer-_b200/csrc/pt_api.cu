@@ -218,7 +218,11 @@ __global__ void k_rng(const uint32_t *tab, uint32_t kind, const uint32_t *pix, c
     Rng r = rng_init(pix[i], npix, smp[i], kind);
     for (uint32_t d = 0; d < dims; d++) out[i * dims + d] = next_float(r, tab);
 }
-__global__ void k_trace_closest(DevScene S, const float *rays, size_t n, pt_hit *out, uint32_t *err) {
+// Ray queries: blocks of 64 rays, 16 per SM (64 registers, the 32 warps of the
+// render's traversal kernels).  A block holds its place until its slowest ray
+// is done, so small blocks keep more warps in flight than blocks of 256 did.
+constexpr unsigned kTraceBlock = 64, kTraceBlocksPerSm = 16;
+__global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSm) k_trace_closest(DevScene S, const float *rays, size_t n, pt_hit *out, uint32_t *err) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *r = rays + 8 * i;
@@ -234,7 +238,7 @@ __global__ void k_trace_closest(DevScene S, const float *rays, size_t n, pt_hit 
     }
     out[i] = o;
 }
-__global__ void k_trace_shadow(DevScene S, const float *rays, size_t n, uint32_t *occ, float *tr, uint32_t *err) {
+__global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSm) k_trace_shadow(DevScene S, const float *rays, size_t n, uint32_t *occ, float *tr, uint32_t *err) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *r = rays + 8 * i;
@@ -972,7 +976,7 @@ int pt_trace_closest(pt_ctx *ctx, const float *rays, size_t n, pt_hit *out, uint
     int rc = s.setup();
     if (rc) return rc;
     cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
-    k_trace_closest<<<blocks_for(n), 256, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (pt_hit *)s.dev(1),
+    k_trace_closest<<<blocks_for(n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (pt_hit *)s.dev(1),
                                                              ctx->d_err);
     rc = s.finish();
     if (rc) return rc;
@@ -994,7 +998,7 @@ int pt_trace_shadow(pt_ctx *ctx, const float *rays, size_t n, uint32_t *occ, flo
     int rc = s.setup();
     if (rc) return rc;
     cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
-    k_trace_shadow<<<blocks_for(n), 256, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (uint32_t *)s.dev(1),
+    k_trace_shadow<<<blocks_for(n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (uint32_t *)s.dev(1),
                                                             (float *)s.dev(2), ctx->d_err);
     rc = s.finish();
     if (rc) return rc;

@@ -347,15 +347,12 @@ __device__ __forceinline__ void bind_stack(TravStack &, uint2 *) {}
     QueueStack<kSharedStack>::type K;                                    \
     bind_stack(K, &stk_[0][threadIdx.x]);
 
-// Traversal kernels run 4 blocks of 256 threads per SM (64 registers).  The
-// opaque-scene forms fit that by themselves (and are left to the compiler:
-// the same bound stated explicitly schedules them worse); the media forms
-// (free flight after the closest hit, ratio tracking on shadow rays) would
-// take 80 registers and 3 blocks, so their entry points state the bound —
-// their traversal waits on DRAM in large scenes and wants the warps more than
-// those registers.
+// Traversal kernels run 4 blocks of 256 threads per SM (64 registers).  Left
+// to the compiler the opaque-scene forms take 70 registers and 3 blocks
+// (64-sphere frame: extend 15.66 against 14.43 ms) and the media forms (free
+// flight after the closest hit, ratio tracking on shadow rays) 80; traversal
+// wants the fourth block's warps more than those registers.
 constexpr int kTraversalBlocksPerSm = 4;
-
 
 // Persistent work-stealing over a ray queue: each warp claims the next 32
 // queue positions with one atomic (so a warp's rays stay neighbours in the
@@ -427,7 +424,7 @@ __device__ __forceinline__ void extend_queue(const WaveArgs &A) {
     }
 }
 template <bool CLASSIFY>
-__global__ void __launch_bounds__(kBlock) k_extend(WaveArgs A) {
+__global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_extend(WaveArgs A) {
     extend_queue<CLASSIFY, false>(A);
 }
 __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_extend_media(WaveArgs A) {
@@ -488,7 +485,7 @@ __device__ __forceinline__ void shadow_queue(const WaveArgs &A) {
         if (i < n) shadow_one<MEDIA_TR>(A, i, K);
     }
 }
-__global__ void __launch_bounds__(kBlock) k_shadow(WaveArgs A) { shadow_queue<false>(A); }
+__global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_shadow(WaveArgs A) { shadow_queue<false>(A); }
 __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_shadow_media(WaveArgs A) {
     shadow_queue<true>(A);
 }
