@@ -665,10 +665,11 @@ __device__ __forceinline__ RayPre ray_pre(float3 o, float3 d) {
     return r;
 }
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, uint32_t i) { return (w >> (8u * i)) & 0xFFu; }
-// Byte `i` of w in the second mantissa byte of 1.0: the float 1 + byte * 2^-15,
-// built by one byte permute (ALU) instead of a conversion (XU).
-__device__ __forceinline__ float byte_in_one(uint32_t w, uint32_t i) {
-    return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | (i << 4)));
+// Byte `i` of w in the low mantissa byte of 2^23: the float 2^23 + byte, built
+// by one byte permute (ALU); subtracting 2^23 (FMA pipe) leaves (float)byte
+// exactly, as the conversion (XU) gives it.
+__device__ __forceinline__ float byte_in_2p23(uint32_t w, uint32_t i) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | i));
 }
 
 // Three-input float max / min (PTX 8.8, sm_100): the same value as two
@@ -699,26 +700,28 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     return d;
 }
 
-// Offsets of the near and far planes of an axis decoded by byte_in_one: with
-// s = 2^15 x the plane step, t = (1 + byte 2^-15) s + (o - s).  Rounding o - s
-// costs up to 2^-9 of a grid step, so the near planes move out by 2^-7 of a
-// step and the far planes by as much: the box test stays conservative.
-__device__ __forceinline__ unsigned long long plane_offsets(float o, float s) {
-    const float q = o - s, pad = fabsf(s);
-    return pack2(fmaf(pad, -2.384185791015625e-7f, q), fmaf(pad, 2.384185791015625e-7f, q));  // 2^-22
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 // Intersect the 8 children of node `ni`: internal hits (in near-to-far visit
 // order, bit k = slot k ^ oct) into gHits, triangle hits into tHits.
 //
 // Bound by instruction issue (72 % of the slots at 4 blocks per SM) and close
 // to that by the ALU and the conversion unit, so the work is spread over the
-// pipes: x and y planes by byte permute (ALU), z planes by conversion (XU),
-// each child's near and far plane of an axis in one packed FMA, the eight
-// comparisons as sign bits shifted into one word, and the triangle bits only
-// for the leaf children that were hit.  Against one FMA per plane and a hit
-// mask assembled for every child (64-sphere frame, 64 spp): extend 15.69 ->
-// 14.43 ms, shadow 5.20 -> 4.63 ms; all planes by permute 14.75 / 4.85, only
-// x by permute 15.76 / 5.25.
+// pipes: x planes and half of the y planes by conversion (XU), the others by
+// byte permute (ALU) and an exact packed subtraction, a child's near and far
+// plane of an axis in one packed FMA, the eight comparisons as sign bits
+// shifted into one word, and triangle bits only for the leaf children hit.
+// Against one FMA per plane and a hit mask assembled for every child
+// (64-sphere frame, 64 spp): extend 15.69 -> 14.46 ms, shadow 5.18 -> 4.74;
+// conversions for x only 14.68 / 4.82, for x and y 14.69 / 4.83, for none
+// 15.21 / 4.90.  Every plane distance and comparison rounds as the unpacked
+// form's, so the same boxes are entered and, where two triangles tie at one
+// t, the same one of them is found.  (Folding the 2^23 into the offset with
+// padded boxes is cheaper, 14.35 / 4.48 ms, but enters a few boxes more: one
+// pixel in some 8 frames of 59 M paths took the other triangle of a tie.)
 __device__ __forceinline__ void intersect_node(const DevScene &S, uint32_t ni, const RayPre &r, float tmin, float tmax,
                                                uint32_t &gBase, uint32_t &gImask, uint32_t &gHits, uint32_t &tBase,
                                                uint32_t &tHits) {
@@ -736,26 +739,28 @@ __device__ __forceinline__ void intersect_node(const DevScene &S, uint32_t ni, c
     if (r.idir.x < 0.0f) { uint32_t t0 = lxa, t1 = lxb; lxa = hxa; lxb = hxb; hxa = t0; hxb = t1; }
     if (r.idir.y < 0.0f) { uint32_t t0 = lya, t1 = lyb; lya = hya; lyb = hyb; hya = t0; hyb = t1; }
     if (r.idir.z < 0.0f) { uint32_t t0 = lza, t1 = lzb; lza = hza; lzb = hzb; hza = t0; hzb = t1; }
-    const float sx = __uint_as_float((ex + 15u) << 23) * r.idir.x;  // 2^15 x the plane step
-    const float sy = __uint_as_float((ey + 15u) << 23) * r.idir.y;
-    const float sz = __uint_as_float(ez << 23) * r.idir.z;
-    const float oz = (pz - r.o.z) * r.idir.z;
-    const unsigned long long Ox = plane_offsets((px - r.o.x) * r.idir.x, sx),
-                             Oy = plane_offsets((py - r.o.y) * r.idir.y, sy), Oz = pack2(oz, oz);
+    const float sx = __uint_as_float(ex << 23) * r.idir.x, ox = (px - r.o.x) * r.idir.x;
+    const float sy = __uint_as_float(ey << 23) * r.idir.y, oy = (py - r.o.y) * r.idir.y;
+    const float sz = __uint_as_float(ez << 23) * r.idir.z, oz = (pz - r.o.z) * r.idir.z;
     const unsigned long long Sx = pack2(sx, sx), Sy = pack2(sy, sy), Sz = pack2(sz, sz);
+    const unsigned long long Ox = pack2(ox, ox), Oy = pack2(oy, oy), Oz = pack2(oz, oz);
+    const unsigned long long m23 = pack2(-8388608.0f, -8388608.0f);
     uint32_t miss = 0;
+    auto planes = [&](uint32_t wn, uint32_t wf, uint32_t sel, bool cvt) {
+        return cvt ? pack2((float)byte_of(wn, sel), (float)byte_of(wf, sel))
+                   : add2(pack2(byte_in_2p23(wn, sel), byte_in_2p23(wf, sel)), m23);
+    };
 #pragma unroll
     for (int i = 7; i >= 0; i--) {
         const uint32_t sel = i & 3u;
         float tnx, tfx, tny, tfy, tnz, tfz;
-        unpack2(fma2(pack2(byte_in_one(i < 4 ? lxa : lxb, sel), byte_in_one(i < 4 ? hxa : hxb, sel)), Sx, Ox), tnx, tfx);
-        unpack2(fma2(pack2(byte_in_one(i < 4 ? lya : lyb, sel), byte_in_one(i < 4 ? hya : hyb, sel)), Sy, Oy), tny, tfy);
-        unpack2(fma2(pack2((float)byte_of(i < 4 ? lza : lzb, sel), (float)byte_of(i < 4 ? hza : hzb, sel)), Sz, Oz), tnz,
-                tfz);
+        unpack2(fma2(planes(i < 4 ? lxa : lxb, i < 4 ? hxa : hxb, sel, true), Sx, Ox), tnx, tfx);
+        unpack2(fma2(planes(i < 4 ? lya : lyb, i < 4 ? hya : hyb, sel, i < 4), Sy, Oy), tny, tfy);
+        unpack2(fma2(planes(i < 4 ? lza : lzb, i < 4 ? hza : hzb, sel, false), Sz, Oz), tnz, tfz);
         const float t0 = fmax3(tnx, tny, fmaxf(tnz, tmin));
         const float t1 = fmin3(tfx, tfy, fminf(tfz, tmax));
-        // missed where t0 > t1 (1 + 2^-22): the difference's sign bit
-        miss = __funnelshift_l(__float_as_uint(fmaf(t1, 1.00000024f, -t0)), miss, 1);
+        // missed where t0 > t1 x (1 + 2^-22): the difference's sign bit
+        miss = __funnelshift_l(__float_as_uint(__fadd_rn(__fmul_rn(t1, 1.00000024f), -t0)), miss, 1);
     }
     const uint32_t hit = ~miss & 0xFFu;
     // internal children: bit i to bit i ^ oct by three conditional swaps
