@@ -300,6 +300,7 @@ int pt_destroy(pt_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     pt_graph_free(ctx);
     pt_batch_free(ctx);
+    pt_branch_free(ctx);
     ctx->free_scene();
     pt_wave_free(ctx);
     if (ctx->scratch) cudaFree(ctx->scratch);

@@ -59,14 +59,18 @@ __host__ __device__ inline int shade_class(bool hit, bool emitter, uint32_t type
     return textured ? c + CLS_TEX : c;
 }
 
-// Words of the per-wave counter block (WaveBuffers::counters).  The claim
-// positions of the work-stealing traversal kernels sit right after the
-// counts that are zeroed together with them each bounce: the shadow count
-// (word 2) and the class counts (words 8 .. 8 + CLS_N).
+// Counters (WaveBuffers::counters) in blocks of kCounterWords words.  Block 0
+// belongs to the render: [4..7] total extension / shadow rays (two uint64),
+// [kCntTailRays] the tail's, [kCntRest].  Block 1 + b belongs to bounce b of the running
+// wave: [0] its ray count, [kCntShadow] its shadow rays, the claim positions
+// of the work-stealing traversal kernels and its shading-class counts.  With
+// a block per bounce one memset clears a whole wave's counters, and a
+// bounce's shadow kernel can still run while the next bounce has begun.
 constexpr int kCounterWords = 32;
 constexpr int kCntShadow = 2, kCntStealExt = 3, kCntClass = 8, kCntStealShadow = kCntClass + CLS_N;
 constexpr int kCntTailRays = 24;  // uint64: extension rays of the tail kernel
-static_assert(kCntStealShadow + 1 <= kCntTailRays && kCntTailRays + 2 <= kCounterWords,
+constexpr int kCntRest = 26;      // kernels of the conditional bodies that ran
+static_assert(kCntStealShadow + 1 <= kCntTailRays && kCntRest + 1 <= kCounterWords,
               "class queue counts and the tail's ray count must fit the counter block");
 
 // Per-wave buffers of the wavefront integrator (structure of arrays).
@@ -87,11 +91,9 @@ struct WaveBuffers {
     // shadow queue (two per path per bounce at most)
     uint32_t *sslot = nullptr;           // slot | kind << 31
     float4 *so = nullptr, *sd = nullptr, *sX = nullptr, *sthr = nullptr;
-    // counters: [0] ray count q0, [1] ray count q1, [2] shadow count, [3]
-    // k_extend claim position, [4..7] total extension / shadow rays (two
-    // uint64), [8 .. 8+CLS_N) class queue counts, [8+CLS_N] k_shadow claim
-    // position; kCounterWords words in all
+    // counter blocks (kCounterWords each): the render's, then one per bounce
     uint32_t *counters = nullptr;
+    size_t counterBounces = 0;
 };
 
 // A render's launch sequence captured as a CUDA graph, with the configuration
@@ -177,6 +179,13 @@ struct pt_ctx {
     // before every render: after the upload, or on the render stream)
     cudaStream_t copyStream = nullptr;
     cudaEvent_t filmReady = nullptr, streamMark = nullptr;
+    // branches of a captured render (ForkJoin in pt_render.cu): streams and
+    // events that take part in captures only; [1]: of a conditional node's
+    // body, which is a capture of its own on bodyStream
+    static constexpr int kBranches = 6;
+    cudaStream_t branch[2][kBranches] = {}, bodyStream = nullptr;
+    cudaEvent_t forkEv[2] = {}, joinEv[2][kBranches] = {};
+    bool branchesReady = false;
     std::string err;
     std::vector<void *> sceneAllocs;  // freed on re-upload / destroy
     pt::DevScene S{};
@@ -300,4 +309,5 @@ cudaError_t rc_enqueue_targets(pt_ctx *ctx, cudaStream_t st, float4 *lo_eta, uin
 cudaError_t rc_enqueue_train(pt_ctx *ctx, cudaStream_t st, uint32_t s, bool adam);
 constexpr uint32_t kRcStepsPerCall = 4;  // Adam steps per cached render call, on interleaved quarters of its records
 void pt_graph_free(pt_ctx *ctx);
+void pt_branch_free(pt_ctx *ctx);
 void pt_batch_free(pt_ctx *ctx);

@@ -74,6 +74,7 @@ struct WaveArgs {
     uint32_t clsStride;
     unsigned long long *rayTotals;  // [0] extension, [1] shadow
     unsigned long long *tailRays;   // extension rays of k_tail (also in rayTotals[0])
+    uint32_t *restLaunched;         // kernels launched by the conditional bodies after k_tail
     uint32_t tailMax;               // k_tail takes a wave's paths when at most this many are left
     uint32_t *err;
     uint32_t shadowCap;
@@ -349,7 +350,8 @@ __device__ __forceinline__ void bind_stack(TravStack &, uint2 *) {}
 
 // Traversal kernels run 4 blocks of 256 threads per SM (64 registers).  Left
 // to the compiler the opaque-scene forms take 70 registers and 3 blocks
-// (64-sphere frame: extend 15.66 against 14.43 ms) and the media forms (free
+// (64-sphere frame, an earlier form of the node test: extend 15.66 against
+// 14.43 ms) and the media forms (free
 // flight after the closest hit, ratio tracking on shadow rays) 80; traversal
 // wants the fourth block's warps more than those registers.
 constexpr int kTraversalBlocksPerSm = 4;
@@ -392,11 +394,9 @@ __device__ __forceinline__ void extend_one(const WaveArgs &A, uint32_t i, Stack 
         uint32_t svi;
         bool sc = sample_free_flight(A.S, make_float3(o.x, o.y, o.z), make_float3(d.x, d.y, d.z),
                                      h.gid != 0xFFFFFFFFu ? h.t : 1e20f, r, vw, tsc, svi);
-        if (r.dim != st.x || r.white != st.y) {
-            st.x = r.dim;
-            st.y = r.white;
-            A.rng[slot] = st;
-        }
+        // only the two words that change: the previous bounce's shadow kernel
+        // may be reading the path's bounce beside this kernel
+        if (r.dim != st.x || r.white != st.y) *reinterpret_cast<uint2 *>(A.rng + slot) = make_uint2(r.dim, r.white);
         if (vw.x != 1.0f || vw.y != 1.0f || vw.z != 1.0f) {
             float4 tp = A.thr_pdf[slot];
             float3 t3 = make_float3(tp.x, tp.y, tp.z) * vw;
@@ -440,7 +440,7 @@ __device__ __forceinline__ void shadow_one(const WaveArgs &A, uint32_t i, Stack 
     uint32_t aseed = 0, akey = 0;
     if (A.S.hasAlpha) {  // the shading kernel already advanced the path's bounce counter
         uint32_t s = A.sslot[i], slot = s & kShadowSlotMask;
-        Rng r = load_rng(A, slot, A.rng[slot]);
+        Rng r = load_rng(A, slot, make_uint4(0u, 0u, 0u, 0u));  // seeds only
         aseed = alpha_seed(r.pixelSeed, r.sampleIndex);
         akey = alpha_key(A.rng[slot].z - 1u, (s >> 31) ? 2u : 1u);
     }
@@ -454,7 +454,7 @@ __device__ __forceinline__ void shadow_one(const WaveArgs &A, uint32_t i, Stack 
         // estimated only now that the ray is known to be unoccluded: its own
         // white-noise stream, keyed by pixel, sample, bounce and NEE kind.  The
         // shading kernel integrated to the light (area: tmax + 0.001)
-        Rng r = load_rng(A, slot, A.rng[slot]);
+        Rng r = load_rng(A, slot, make_uint4(0u, 0u, 0u, 0u));  // seeds only
         Rng t;
         t.kind = PT_RNG_PCG_HASH;
         t.pixelSeed = r.pixelSeed;
@@ -1404,9 +1404,17 @@ __global__ void __launch_bounds__(kBlock, 2) k_tail(WaveArgs A) {
     for (int o = 16; o > 0; o >>= 1) ext += __shfl_xor_sync(0xFFFFFFFFu, ext, o);
     if (lane_id() == 0 && ext) atomicAdd(A.tailRays, (unsigned long long)ext);
 }
-// After k_tail: if it ran, its paths are done and the queue is empty.
-__global__ void k_tail_close(WaveArgs A) {
-    if (*A.cntIn <= A.tailMax) *A.cntIn = 0u;
+// After k_tail: if it ran, its paths are done and the queue is empty.  In a
+// captured render the bounces that follow are the body of a conditional node,
+// which runs only when k_tail left them to do (`rest`, 0: no such node;
+// restLaunches: the kernels of that body).
+__global__ void k_tail_close(WaveArgs A, cudaGraphConditionalHandle rest, uint32_t restLaunches) {
+    const bool done = *A.cntIn <= A.tailMax;
+    if (done) *A.cntIn = 0u;
+    if (rest) {
+        cudaGraphSetConditional(rest, done ? 0u : 1u);
+        if (!done) *A.restLaunched += restLaunches;
+    }
 }
 
 // ---- film: Kahan-compensated accumulation of (L, 1), samples in order -------
@@ -1538,7 +1546,6 @@ static int wave_alloc(pt_ctx *ctx, size_t cap) {
     A((void **)&W.cls, cap * 4 * CLS_N);
     A((void **)&W.sslot, sc * 4); A((void **)&W.so, sc * 16); A((void **)&W.sd, sc * 16);
     A((void **)&W.sX, sc * 16); A((void **)&W.sthr, sc * 16);
-    A((void **)&W.counters, kCounterWords * sizeof(uint32_t));
     if (e != cudaSuccess) {
         pt_wave_free(ctx);
         return ctx->fail(PT_E_NOMEM, "wave buffers", cudaGetErrorString(e));
@@ -1588,6 +1595,54 @@ inline uint32_t tail_bounce(uint32_t depth, const WaveArgs &A, uint32_t tailMode
 }
 struct Mark { int stage; cudaEvent_t a, b; };
 
+// Counter blocks for renders of up to `depth` bounces.
+int counters_alloc(pt_ctx *ctx, uint32_t depth) {
+    WaveBuffers &W = ctx->W;
+    const size_t want = std::max<size_t>(depth, 32) + 1;  // a block for the queue the last bounce leaves, too
+    if (W.counters && W.counterBounces >= want) return PT_OK;
+    if (W.counters) cudaFree(W.counters);
+    W.counters = nullptr;
+    W.counterBounces = 0;
+    cudaError_t e = cudaMalloc((void **)&W.counters, (1 + want) * kCounterWords * sizeof(uint32_t));
+    if (e != cudaSuccess) return ctx->fail(PT_E_NOMEM, "wave counters", cudaGetErrorString(e));
+    W.counterBounces = want;
+    ctx->waveGen++;
+    return PT_OK;
+}
+
+// Parallel branches of a captured render.  Within a bounce the shading
+// kernels of the classes are independent of one another, and the shadow
+// kernel is independent of the next bounce's closest-hit kernel (both write
+// results that only the next shading pass reads), so in a graph they are
+// parallel nodes: with few paths each kernel lasts as long as its slowest
+// thread, and a bounce then costs two such times instead of one per kernel.
+// Measured, one stream -> branches (with one memset per wave instead of three
+// per bounce, the conditional body and the launch shapes below): 64 x 64 room
+// 0.75 -> 0.40 ms, 1280 x 720 preview 1.91 -> 1.41 ms, fog scene at 1917 x
+// 1079 x 4 17.4 -> 15.5 ms, 59 M-path frame 27.2 -> 26.9 ms.
+struct ForkJoin {
+    const cudaStream_t *branch;
+    cudaEvent_t forkEv;
+    const cudaEvent_t *joinEv;
+};
+bool branches_ready(pt_ctx *ctx) {
+    if (ctx->branchesReady) return true;
+    bool ok = cudaStreamCreateWithFlags(&ctx->bodyStream, cudaStreamNonBlocking) == cudaSuccess;
+    for (int k = 0; k < 2; k++) {
+        ok = ok && cudaEventCreateWithFlags(&ctx->forkEv[k], cudaEventDisableTiming) == cudaSuccess;
+        for (int i = 0; i < pt_ctx::kBranches; i++) {
+            ok = ok && cudaStreamCreateWithFlags(&ctx->branch[k][i], cudaStreamNonBlocking) == cudaSuccess;
+            ok = ok && cudaEventCreateWithFlags(&ctx->joinEv[k][i], cudaEventDisableTiming) == cudaSuccess;
+        }
+    }
+    if (!ok) {
+        cudaGetLastError();
+        pt_branch_free(ctx);
+    }
+    ctx->branchesReady = ok;
+    return ok;
+}
+
 // Issues one render's work on a stream: directly (optionally with an event
 // pair around every launch), or into a stream capture.
 struct Enqueue {
@@ -1595,6 +1650,7 @@ struct Enqueue {
     bool timing;
     std::vector<Mark> marks;
     uint64_t launches = 0;
+    const ForkJoin *fj = nullptr;  // set in captures: issue independent kernels as parallel branches
     void begin(int stage) {
         launches++;
         if (!timing) return;
@@ -1616,9 +1672,91 @@ struct Grids {
     int tail, tailI;
 };
 
+// Launch shape of a kernel that loops over a queue of at most `n` entries of
+// a wave of `paths`: the resident grid, or no more blocks than entries; in
+// blocks of 64 when the wave's paths are resident at once anyway (1024 per
+// SM): its threads then spread over all SMs instead of filling a few.
+struct Shape { unsigned grid, block; };
+inline Shape queue_shape(int grid, uint64_t n, uint64_t paths, int numSMs) {
+    const unsigned block = paths <= (uint64_t)numSMs * 1024u ? 64u : (unsigned)kBlock;
+    return {(unsigned)std::min<uint64_t>((n + block - 1) / block, (uint64_t)grid * (kBlock / block)), block};
+}
+// Kernels per bounce of a wave (launch counts).
+inline uint32_t bounce_launches(const pt_ctx *ctx, const WaveArgs &A) {
+    if ((ctx->S.numVols > 0 && !A.S.mediaWavefront) || ctx->S.hasSubsurface) return 2;
+    return 2 + (uint32_t)__builtin_popcount(ctx->clsMask | (A.S.mediaWavefront ? 1u << CLS_MEDIUM : 0u));
+}
+
+cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t first, uint32_t depth,
+                            const Grids &G, bool tail);
+
+// In a capture: k_tail_close and the bounces after the tail kernel as the body
+// of a conditional node that it opens when paths are left.  (Launched
+// unconditionally, the empty kernels of 12 bounces were 0.25 ms of every
+// render whose paths the tail had finished.)  False: no conditional node can
+// be made here and nothing was added to the capture.
+bool enqueue_rest_conditional(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t first, uint32_t depth,
+                              const Grids &G, cudaError_t &err) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo_v2(E.st, &cs, nullptr, &graph) != cudaSuccess || cs != cudaStreamCaptureStatusActive)
+        return false;
+    cudaGraphConditionalHandle h = 0;
+    if (cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    k_tail_close<<<1, 1, 0, E.st>>>(A, h, (depth - first) * bounce_launches(ctx, A));
+    auto chk = [&](cudaError_t e) {
+        if (err == cudaSuccess && e != cudaSuccess) err = e;
+    };
+    const cudaGraphNode_t *deps = nullptr;
+    size_t nd = 0;
+    chk(cudaStreamGetCaptureInfo_v2(E.st, &cs, nullptr, &graph, &deps, &nd));
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = h;
+    np.conditional.type = cudaGraphCondTypeIf;
+    np.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    if (err == cudaSuccess) chk(cudaGraphAddNode(&node, graph, deps, nd, &np));
+    if (err != cudaSuccess) return true;
+    chk(cudaStreamUpdateCaptureDependencies(E.st, &node, 1, cudaStreamSetCaptureDependencies));
+    cudaGraph_t body = np.conditional.phGraph_out[0];
+    chk(cudaStreamBeginCaptureToGraph(ctx->bodyStream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    if (err != cudaSuccess) return true;
+    const cudaStream_t outer = E.st;
+    const ForkJoin *const outerFj = E.fj;
+    const ForkJoin fj{ctx->branch[1], ctx->forkEv[1], ctx->joinEv[1]};
+    const uint64_t launches = E.launches;  // the body's count when it runs (k_tail_close)
+    E.st = ctx->bodyStream;
+    E.fj = &fj;
+    chk(enqueue_bounces(ctx, E, A, first, depth, G, false));
+    chk(cudaStreamEndCapture(E.st, &body));
+    E.st = outer;
+    E.fj = outerFj;
+    E.launches = launches;
+    return true;
+}
+
 // Raygen and `depth` bounces of one wave (A.waveStart / A.waveCount set).
 // Returns the first failing call's status (cudaSuccess if none).
 cudaError_t enqueue_paths(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t depth, const Grids &G) {
+    const WaveBuffers &B = ctx->W;
+    // the counters of every bounce of the wave
+    cudaError_t err = cudaMemsetAsync(B.counters + kCounterWords, 0,
+                                      ((size_t)depth + 1) * kCounterWords * sizeof(uint32_t), E.st);
+    A.qslotOut = B.qslot[0]; A.qoOut = B.qo[0]; A.qdOut = B.qd[0]; A.cntOut = B.counters + kCounterWords;
+    E.begin(STG_RAYGEN);
+    k_raygen<<<(A.waveCount + kBlock - 1) / kBlock, kBlock, 0, E.st>>>(A);
+    E.end();
+    const cudaError_t e = enqueue_bounces(ctx, E, A, 0, depth, G, true);
+    return err != cudaSuccess ? err : e;
+}
+
+// Bounces [first, depth) of a wave; `tail`: the tail kernel may take over.
+cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t first, uint32_t depth,
+                            const Grids &G, bool tail) {
     const WaveBuffers &B = ctx->W;
     const bool inl = (ctx->S.numVols > 0 && !A.S.mediaWavefront) || ctx->S.hasSubsurface;
     cudaStream_t st = E.st;
@@ -1626,55 +1764,103 @@ cudaError_t enqueue_paths(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t d
     auto chk = [&](cudaError_t e) {
         if (err == cudaSuccess && e != cudaSuccess) err = e;
     };
-    A.qslotOut = B.qslot[0]; A.qoOut = B.qo[0]; A.qdOut = B.qd[0]; A.cntOut = B.counters + 0;
-    E.begin(STG_RAYGEN);
-    k_raygen<<<(A.waveCount + kBlock - 1) / kBlock, kBlock, 0, st>>>(A);
-    E.end();
-    int cur = 0;
-    for (uint32_t b = 0; b < depth; b++) {
+    const ForkJoin *fj = E.fj;
+    bool shadowOpen = false;  // the previous bounce's shadow kernel runs on branch 0
+    auto joinShadow = [&]() {
+        if (shadowOpen) chk(cudaStreamWaitEvent(st, fj->joinEv[0], 0));
+        shadowOpen = false;
+    };
+    for (uint32_t b = first; b < depth; b++) {
+        const int cur = (int)(b & 1u);
+        uint32_t *cnt = B.counters + (size_t)(1 + b) * kCounterWords;
         A.bounce = b;
-        A.qslotIn = B.qslot[cur]; A.qoIn = B.qo[cur]; A.qdIn = B.qd[cur]; A.cntIn = B.counters + cur;
+        A.qslotIn = B.qslot[cur]; A.qoIn = B.qo[cur]; A.qdIn = B.qd[cur]; A.cntIn = cnt;
         A.qslotOut = B.qslot[1 - cur]; A.qoOut = B.qo[1 - cur]; A.qdOut = B.qd[1 - cur];
-        A.cntOut = B.counters + (1 - cur);
-        chk(cudaMemsetAsync(A.cntOut, 0, 4, st));
-        chk(cudaMemsetAsync(A.cntShadow, 0, 8, st));  // shadow count and the extend claim position
-        if (b == tail_bounce(depth, A, ctx->dbgTail)) {  // the remaining bounces of every path in one launch, when few are left
+        A.cntOut = cnt + kCounterWords;
+        A.cntShadow = cnt + kCntShadow;
+        A.stealExt = cnt + kCntStealExt;
+        A.stealShadow = cnt + kCntStealShadow;
+        A.cntCls = cnt + kCntClass;
+        auto shape = [&](int grid, uint64_t n) { return queue_shape(grid, n, A.waveCount, ctx->numSMs); };
+        if (tail && b == tail_bounce(depth, A, ctx->dbgTail)) {  // the remaining bounces of every path in one launch, when few are left
+            joinShadow();
             E.begin(STG_TAIL);
             if (inl) k_tail<true><<<G.tailI, kBlock, 0, st>>>(A);
             else k_tail<false><<<G.tail, kBlock, 0, st>>>(A);
-            k_tail_close<<<1, 1, 0, st>>>(A);
+            if (fj) {
+                if (enqueue_rest_conditional(ctx, E, A, b, depth, G, err)) return err;
+            }
+            k_tail_close<<<1, 1, 0, st>>>(A, 0, 0u);
             E.end();
+            if (E.timing) {  // stage by stage: the host reads what the conditional node would
+                uint32_t left = 1;
+                chk(cudaMemcpyAsync(&left, A.cntIn, sizeof(left), cudaMemcpyDeviceToHost, st));
+                chk(cudaStreamSynchronize(st));
+                if (err == cudaSuccess && left == 0u) return err;
+            }
         }
         if (inl) {
+            const Shape x = shape(G.ext, A.waveCount), h = shape(G.shadeI, A.waveCount);
             E.begin(STG_EXTEND);
-            k_extend<false><<<G.ext, kBlock, 0, st>>>(A);
+            k_extend<false><<<x.grid, x.block, 0, st>>>(A);
             E.end();
             E.begin(STG_SHADE);
-            k_shade<true, CLS_ANY><<<G.shadeI, kBlock, 0, st>>>(A);
+            k_shade<true, CLS_ANY><<<h.grid, h.block, 0, st>>>(A);
             E.end();
+            continue;
+        }
+        E.begin(STG_EXTEND);
+        if (A.S.mediaWavefront) {
+            const Shape x = shape(G.extM, A.waveCount);
+            k_extend_media<<<x.grid, x.block, 0, st>>>(A);
         } else {
-            // class counts and the shadow claim position after them
-            chk(cudaMemsetAsync(A.cntCls, 0, (CLS_N + 1) * sizeof(uint32_t), st));
-            E.begin(STG_EXTEND);
-            if (A.S.mediaWavefront) k_extend_media<<<G.extM, kBlock, 0, st>>>(A);
-            else k_extend<true><<<G.extC, kBlock, 0, st>>>(A);
-            E.end();
-            const bool extra = A.risNee || A.S.mediaWavefront;
-            const uint32_t mask = ctx->clsMask | (A.S.mediaWavefront ? 1u << CLS_MEDIUM : 0u);
-            for (int c = 0; c < CLS_N; c++) {
-                if (!((mask >> c) & 1u)) continue;
-                E.begin(STG_SHADE);
-                if (extra) kShadeClsX[c]<<<G.clsX[c], kBlock, 0, st>>>(A);
-                else kShadeCls[c]<<<G.cls[c], kBlock, 0, st>>>(A);
-                E.end();
+            const Shape x = shape(G.extC, A.waveCount);
+            k_extend<true><<<x.grid, x.block, 0, st>>>(A);
+        }
+        E.end();
+        joinShadow();  // the shading pass folds its results in
+        const bool extra = A.risNee || A.S.mediaWavefront;
+        const uint32_t mask = ctx->clsMask | (A.S.mediaWavefront ? 1u << CLS_MEDIUM : 0u);
+        if (fj) chk(cudaEventRecord(fj->forkEv, st));
+        uint32_t used = 0;  // branches with shading kernels of this bounce
+        int k = 0;
+        for (int c = 0; c < CLS_N; c++) {
+            if (!((mask >> c) & 1u)) continue;
+            cudaStream_t cs = st;
+            const int br = k++ % (pt_ctx::kBranches + 1) - 1;  // the first class on the main branch
+            if (fj && br >= 0) {
+                cs = fj->branch[br];
+                if (!((used >> br) & 1u)) chk(cudaStreamWaitEvent(cs, fj->forkEv, 0));
+                used |= 1u << br;
             }
-            E.begin(STG_SHADOW);
-            if (A.S.mediaTrDeferred) k_shadow_media<<<G.shadowM, kBlock, 0, st>>>(A);
-            else k_shadow<<<G.shadow, kBlock, 0, st>>>(A);
+            const Shape h = shape(extra ? G.clsX[c] : G.cls[c], A.waveCount);
+            E.begin(STG_SHADE);
+            if (extra) kShadeClsX[c]<<<h.grid, h.block, 0, cs>>>(A);
+            else kShadeCls[c]<<<h.grid, h.block, 0, cs>>>(A);
             E.end();
         }
-        cur = 1 - cur;
+        for (int br = 0; br < pt_ctx::kBranches; br++)
+            if ((used >> br) & 1u) {
+                chk(cudaEventRecord(fj->joinEv[br], fj->branch[br]));
+                chk(cudaStreamWaitEvent(st, fj->joinEv[br], 0));
+            }
+        cudaStream_t ss = st;
+        if (fj) {  // beside the next bounce's closest-hit kernel
+            ss = fj->branch[0];
+            chk(cudaEventRecord(fj->forkEv, st));
+            chk(cudaStreamWaitEvent(ss, fj->forkEv, 0));
+        }
+        const Shape w = shape(A.S.mediaTrDeferred ? G.shadowM : G.shadow, 2ull * A.waveCount);
+        E.begin(STG_SHADOW);
+        if (A.S.mediaTrDeferred) k_shadow_media<<<w.grid, w.block, 0, ss>>>(A);
+        else k_shadow<<<w.grid, w.block, 0, ss>>>(A);
+        E.end();
+        if (fj) {
+            chk(cudaEventRecord(fj->joinEv[0], ss));
+            shadowOpen = true;
+        }
     }
+    joinShadow();
     return err;
 }
 
@@ -1765,6 +1951,22 @@ bool graph_matches(const pt_ctx *ctx, const pt_render_params *P, size_t cap, con
 }
 }  // namespace
 
+void pt_branch_free(pt_ctx *ctx) {
+    for (int k = 0; k < 2; k++) {
+        for (int i = 0; i < pt_ctx::kBranches; i++) {
+            if (ctx->branch[k][i]) cudaStreamDestroy(ctx->branch[k][i]);
+            if (ctx->joinEv[k][i]) cudaEventDestroy(ctx->joinEv[k][i]);
+            ctx->branch[k][i] = nullptr;
+            ctx->joinEv[k][i] = nullptr;
+        }
+        if (ctx->forkEv[k]) cudaEventDestroy(ctx->forkEv[k]);
+        ctx->forkEv[k] = nullptr;
+    }
+    if (ctx->bodyStream) cudaStreamDestroy(ctx->bodyStream);
+    ctx->bodyStream = nullptr;
+    ctx->branchesReady = false;
+}
+
 void pt_graph_free(pt_ctx *ctx) {
     if (ctx->graph.exec) cudaGraphExecDestroy(ctx->graph.exec);
     ctx->graph = RenderGraph{};
@@ -1796,6 +1998,7 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     if (cap > total) cap = (size_t)total;
     if (cap == 0) return PT_OK;
     int rc = wave_alloc(ctx, cap);
+    if (!rc) rc = counters_alloc(ctx, P->max_depth);
     if (rc) return rc;
     cudaStream_t st = ctx->stream;
     WaveBuffers &B = ctx->W;
@@ -1826,14 +2029,11 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     A.thr_pdf = B.thr_pdf; A.lo_eta = B.lo_eta; A.pendA = B.pendA; A.pendE = B.pendE; A.rng = B.rng;
     A.qhit = B.qhit;
     A.sslot = B.sslot; A.so = B.so; A.sd = B.sd; A.sX = B.sX; A.sthr = B.sthr;
-    A.cntShadow = B.counters + kCntShadow;
-    A.stealExt = B.counters + kCntStealExt;
-    A.stealShadow = B.counters + kCntStealShadow;
-    A.cntCls = B.counters + kCntClass;
     A.cls = B.cls;
     A.clsStride = (uint32_t)B.cap;
     A.rayTotals = (unsigned long long *)(B.counters + 4);
     A.tailRays = (unsigned long long *)(B.counters + kCntTailRays);
+    A.restLaunched = B.counters + kCntRest;
     A.tailMax = ctx->dbgTail == 1u ? 0u : kTailMaxPaths;
     A.err = ctx->d_err;
     A.shadowCap = (uint32_t)(2 * B.cap);
@@ -1873,7 +2073,10 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     bool useGraph = !timing;
     if (useGraph && !graph_matches(ctx, P, cap, d_sum, d_comp, A)) {
         pt_graph_free(ctx);
+        const bool forkOk = branches_ready(ctx);
         Enqueue E{ctx->ownStream, false, {}, 0};
+        const ForkJoin fj{ctx->branch[0], ctx->forkEv[0], ctx->joinEv[0]};
+        if (forkOk) E.fj = &fj;
         cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
         bool ok = cudaStreamBeginCapture(ctx->ownStream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
@@ -1947,7 +2150,7 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
         stats->shadow_rays = tot[1];
         stats->waves = waves;
         stats->bounces = waves * P->max_depth;
-        stats->launches = launches;
+        stats->launches = launches + hostCnt[kCntRest];
         stats->ms_total = ms;
         stats->ms_raygen = stage[STG_RAYGEN];
         stats->ms_extend = stage[STG_EXTEND];
@@ -2094,7 +2297,9 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         size_t fit = (freeB / 2 + ctx->W.cap * kWaveBytesPerPath / 2) / (kWaveBytesPerPath + 8);
         cap = std::max<size_t>(std::min(cap, fit), std::min<size_t>(cap, (size_t)1 << 16));
     }
-    if ((rc = wave_alloc(ctx, cap))) return rc;
+    uint32_t deepest = 0;
+    for (uint32_t i = 0; i < n; i++) deepest = std::max(deepest, R[i].params.max_depth);
+    if ((rc = wave_alloc(ctx, cap)) || (rc = counters_alloc(ctx, deepest))) return rc;
     if (Bt.slotCap < cap) {
         if (Bt.slotInfo) cudaFree(Bt.slotInfo);
         Bt.slotInfo = nullptr;
@@ -2186,14 +2391,11 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
     A.thr_pdf = B.thr_pdf; A.lo_eta = B.lo_eta; A.pendA = B.pendA; A.pendE = B.pendE; A.rng = B.rng;
     A.qhit = B.qhit;
     A.sslot = B.sslot; A.so = B.so; A.sd = B.sd; A.sX = B.sX; A.sthr = B.sthr;
-    A.cntShadow = B.counters + kCntShadow;
-    A.stealExt = B.counters + kCntStealExt;
-    A.stealShadow = B.counters + kCntStealShadow;
-    A.cntCls = B.counters + kCntClass;
     A.cls = B.cls;
     A.clsStride = (uint32_t)B.cap;
     A.rayTotals = (unsigned long long *)(B.counters + 4);
     A.tailRays = (unsigned long long *)(B.counters + kCntTailRays);
+    A.restLaunched = B.counters + kCntRest;
     A.tailMax = ctx->dbgTail == 1u ? 0u : kTailMaxPaths;
     A.err = ctx->d_err;
     A.shadowCap = (uint32_t)(2 * B.cap);
@@ -2217,7 +2419,10 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
     if (!Bt.exec || Bt.key != key) {
         if (Bt.exec) cudaGraphExecDestroy(Bt.exec);
         Bt.exec = nullptr;
+        const bool forkOk = branches_ready(ctx);
         Enqueue E{ctx->ownStream, false, {}, 0};
+        const ForkJoin fj{ctx->branch[0], ctx->forkEv[0], ctx->joinEv[0]};
+        if (forkOk) E.fj = &fj;
         cudaGraph_t g = nullptr;
         const char *step = "begin capture";
         cudaError_t ce = cudaStreamBeginCapture(ctx->ownStream, cudaStreamCaptureModeThreadLocal);
@@ -2290,7 +2495,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         uint64_t bounces = 0;
         for (uint32_t d : pl.waveDepth) bounces += d;
         stats->bounces = bounces;
-        stats->launches = Bt.launches;
+        stats->launches = Bt.launches + hostCnt[kCntRest];
         stats->ms_total = ms;
         memcpy(&stats->tail_extension_rays, hostCnt + kCntTailRays, 8);
     }
