@@ -41,10 +41,41 @@ constexpr uint32_t kFlagUnbiased = 8u;  // training path whose suffix does not u
 constexpr uint32_t kFlagHasRec = 16u;   // its training record has been written
 constexpr int kBlock = 256;
 
+// Order of the paths of a render call or of one request of a batch
+// (path_pos_sample): its samples in up to 6 segments of equal groups, segment
+// k holding samples [first[k], first[k + 1]) in groups of 1 << lg[k].
+constexpr int kOrderSegs = 6;
+struct PathOrder {
+    uint32_t npix, fullTilePix;  // pixels; those in full 8 x 4 tiles
+    uint32_t spp, nseg;
+    uint32_t first[kOrderSegs + 1];
+    uint32_t lg[kOrderSegs];
+};
+// fine: groups of 32, then one group for each further bit of spp.  Otherwise
+// (cached renders, whose training records follow the waves' samples): groups
+// of 32, of 8, and single samples.
+inline PathOrder path_order(uint32_t width, uint32_t height, uint32_t spp, bool fine) {
+    PathOrder O{};
+    O.npix = width * height;
+    O.fullTilePix = 32u * (width / 8u) * (height / 4u);
+    O.spp = spp;
+    uint32_t s = 0;
+    for (uint32_t lg : {5u, 4u, 3u, 2u, 1u, 0u}) {
+        const uint32_t n = !fine && (lg == 4u || lg == 2u || lg == 1u) ? 0u : (spp - s) >> lg;
+        if (!n) continue;
+        O.first[O.nseg] = s;
+        O.lg[O.nseg++] = lg;
+        s += n << lg;
+    }
+    for (int k = (int)O.nseg; k <= kOrderSegs; k++) O.first[k] = s;
+    return O;
+}
+
 // One request of a batched render (pt_render_batch), in the device table.
 struct ReqDev {
     uint64_t pathStart;  // first path id of the request in the batch's path order
     uint32_t width, height, npix, spp, sampleOffset, maxDepth;
+    PathOrder ord;
     pt_camera cam;
     float4 *sum, *comp;  // film (device memory)
 };
@@ -52,7 +83,7 @@ struct ReqDev {
 struct WaveArgs {
     DevScene S;
     uint32_t width, height, npix;
-    uint32_t spp, spp32, spp8, fullTilePix;  // the call's samples, those in groups of 32, then of 8; pixels in full 8 x 4 tiles
+    PathOrder ord;  // path order of the call (a batch: of each request, in its table entry)
     uint64_t recKeyBase;  // a training record's order key: sample x npix + position - recKeyBase (this wave)
     uint32_t recKeyRange; // keys of this wave's records lie in [0, recKeyRange)
     const uint32_t *sampleOffset;  // -> sample index of path id 0 of this render call
@@ -143,75 +174,79 @@ __device__ __forceinline__ uint32_t find_request(const WaveArgs &A, uint64_t pid
     }
     return lo;
 }
-// Path order of a render call (path id -> pixel position of tile_pixel,
-// sample of the call).  The call's samples go in groups, so that a warp's
-// 32 paths are camera rays of few pixels: first as many groups of 32 as
-// fit (a warp = 32 samples of one pixel; consecutive warps follow the pixel
-// positions), then groups of 8 (within a group, each 8 x 4 tile's eight
-// 2 x 2 pixel blocks in turn, a block's 32 paths being its 4 pixels x the 8
-// samples; positions outside the full tiles take the group's samples one
-// after the other), and the remaining samples one after the other over the
-// pixel positions.  A bijection; path_id is its inverse (the film sums each
-// pixel's samples in sample order through it).  Measured on the 64-sphere
-// frame (Mpaths/s): one sample at a time 1849, groups of 8 1958, groups of
-// 32 2040; the 10 M-triangle scene at 16 spp per call: 466 -> 489 with 8.
-__host__ __device__ inline void path_pos_sample(const WaveArgs &A, uint64_t pid, uint32_t &p, uint32_t &s) {
-    const uint32_t npix = A.npix;
-    const uint64_t g32 = (uint64_t)A.spp32 * npix;
-    if (pid < g32) {
-        const uint64_t gsz = 32ull * npix;
-        const uint32_t c = (uint32_t)(pid / gsz), r = (uint32_t)(pid % gsz);
-        p = r >> 5;
-        s = 32u * c + (r & 31u);
+// Path order (path id -> pixel position of tile_pixel, sample).  Samples go in
+// groups, so that a warp's 32 paths are camera rays of few pixels: in a group
+// of g samples a warp is 32 / g neighbouring pixels (1, 2 x 1, 2 x 2, 4 x 2,
+// 4 x 4 or the 8 x 4 tile) x the g samples; consecutive warps follow the
+// blocks of a tile, then the tiles.  Positions outside the full tiles take
+// the samples of a group of less than 32 one after the other.  A bijection;
+// path_id is its inverse (the film sums each pixel's samples in sample order
+// through it).  Measured on the 64-sphere frame (Mpaths/s): one sample at a
+// time 1849, groups of 8 1958, groups of 32 2040.
+__host__ __device__ inline void path_pos_sample(const PathOrder &O, uint64_t pid, uint32_t &p, uint32_t &s) {
+    uint32_t k = 0;
+    while (k + 1 < O.nseg && pid >= (uint64_t)O.first[k + 1] * O.npix) k++;
+    const uint32_t lg = O.lg[k];
+    const uint64_t off = pid - (uint64_t)O.first[k] * O.npix, gsz = (uint64_t)O.npix << lg;
+    uint32_t c = 0;
+    uint64_t r = off;
+    if (off >= gsz) {  // not the segment's first group
+        c = ((off | gsz) >> 32) ? (uint32_t)(off / gsz) : (uint32_t)off / (uint32_t)gsz;
+        r = off - c * gsz;
+    }
+    s = O.first[k] + (c << lg);
+    if (lg == 5u) {
+        p = (uint32_t)(r >> 5);
+        s += (uint32_t)r & 31u;
         return;
     }
-    pid -= g32;
-    const uint64_t g8 = (uint64_t)A.spp8 * npix;
-    if (pid < g8) {
-        const uint64_t gsz = 8ull * npix;
-        const uint32_t c = (uint32_t)(pid / gsz), r = (uint32_t)(pid % gsz), full = A.fullTilePix;
-        if (r < 8u * full) {
-            const uint32_t t = r >> 8, q = r & 255u, b = q >> 5, u = q & 31u, i = u & 3u;
-            p = 32u * t + ((2u * (b >> 2) + (i >> 1)) << 3) + 2u * (b & 3u) + (i & 1u);
-            s = A.spp32 + 8u * c + (u >> 2);
-        } else {
-            const uint32_t r2 = r - 8u * full, rem = npix - full;
-            p = full + r2 % rem;
-            s = A.spp32 + 8u * c + r2 / rem;
-        }
-        return;
+    const uint32_t full = O.fullTilePix;
+    if (r < ((uint64_t)full << lg)) {
+        const uint32_t lp = 5u - lg, lw = (lp + 1u) >> 1, lh = lp - lw;  // log2 of a block's pixels, width, height
+        const uint32_t t = (uint32_t)(r >> (5u + lg)), q = (uint32_t)r & ((32u << lg) - 1u), b = q >> 5, u = q & 31u;
+        const uint32_t i = u & ((1u << lp) - 1u), bx = b & ((8u >> lw) - 1u), by = b >> (3u - lw);
+        p = 32u * t + (((by << lh) + (i >> lw)) << 3) + (bx << lw) + (i & ((1u << lw) - 1u));
+        s += u >> lp;
+    } else {
+        const uint64_t r2 = r - ((uint64_t)full << lg);
+        const uint32_t rem = O.npix - full, j = (uint32_t)(r2 / rem);
+        p = full + (uint32_t)(r2 - (uint64_t)j * rem);
+        s += j;
     }
-    const uint64_t q = pid - g8;
-    p = (uint32_t)(q % npix);
-    s = A.spp32 + A.spp8 + (uint32_t)(q / npix);
 }
-__device__ __forceinline__ uint64_t path_id(const WaveArgs &A, uint32_t p, uint32_t s) {
-    const uint32_t npix = A.npix;
-    if (s < A.spp32) return (uint64_t)(s >> 5) * 32u * npix + 32ull * p + (s & 31u);
-    const uint64_t base = (uint64_t)A.spp32 * npix;
-    const uint32_t s2 = s - A.spp32;
-    if (s2 < A.spp8) {
-        const uint64_t gbase = base + (uint64_t)(s2 >> 3) * 8u * npix;
-        const uint32_t si = s2 & 7u, full = A.fullTilePix;
-        if (p < full) {
-            const uint32_t t = p >> 5, w = p & 31u, row = w >> 3, col = w & 7u;
-            return gbase + 256ull * t + 32u * ((row >> 1) * 4u + (col >> 1)) + 4u * si + (row & 1u) * 2u + (col & 1u);
-        }
-        return gbase + 8ull * full + (uint64_t)si * (npix - full) + (p - full);
+__host__ __device__ inline uint64_t path_id(const PathOrder &O, uint32_t p, uint32_t s) {
+    uint32_t k = 0;
+    while (k + 1 < O.nseg && s >= O.first[k + 1]) k++;
+    const uint32_t lg = O.lg[k], j = s - O.first[k], si = j & ((1u << lg) - 1u);
+    const uint64_t gbase = (uint64_t)(O.first[k] + (j - si)) * O.npix;
+    if (lg == 5u) return gbase + 32ull * p + si;
+    const uint32_t full = O.fullTilePix;
+    if (p < full) {
+        const uint32_t lp = 5u - lg, lw = (lp + 1u) >> 1, lh = lp - lw;
+        const uint32_t t = p >> 5, row = (p >> 3) & 3u, col = p & 7u;
+        const uint32_t b = ((row >> lh) << (3u - lw)) + (col >> lw);
+        const uint32_t i = ((row & ((1u << lh) - 1u)) << lw) + (col & ((1u << lw) - 1u));
+        return gbase + ((uint64_t)t << (5u + lg)) + 32u * b + (si << lp) + i;
     }
-    return base + (uint64_t)A.spp8 * npix + (uint64_t)(s2 - A.spp8) * npix + p;
+    return gbase + ((uint64_t)full << lg) + (uint64_t)si * (O.npix - full) + (p - full);
 }
 // The first and last sample of sample s's group.
-__host__ __device__ inline void path_group(const WaveArgs &A, uint32_t s, uint32_t &lo, uint32_t &hi) {
-    if (s < A.spp32) {
-        lo = s & ~31u;
-        hi = s | 31u;
-    } else if (s - A.spp32 < A.spp8) {
-        lo = A.spp32 + ((s - A.spp32) & ~7u);
-        hi = A.spp32 + ((s - A.spp32) | 7u);
-    } else {
-        lo = hi = s;
-    }
+__host__ __device__ inline void path_group(const PathOrder &O, uint32_t s, uint32_t &lo, uint32_t &hi) {
+    uint32_t k = 0;
+    while (k + 1 < O.nseg && s >= O.first[k + 1]) k++;
+    const uint32_t m = (1u << O.lg[k]) - 1u;
+    lo = s - ((s - O.first[k]) & m);
+    hi = lo + m;
+}
+// The samples that the paths [first, last) can hold: those of the first and
+// last path, widened to their groups.
+__host__ __device__ inline void path_samples(const PathOrder &O, uint64_t first, uint64_t last, uint32_t &s0,
+                                             uint32_t &s1) {
+    uint32_t p, lo, hi;
+    path_pos_sample(O, first, p, s0);
+    path_pos_sample(O, last - 1, p, s1);
+    path_group(O, s0, s0, hi);
+    path_group(O, s1, lo, s1);
 }
 __device__ __forceinline__ void path_coords(const WaveArgs &A, uint32_t slot, uint32_t &pix, uint32_t &frame) {
     if (A.batch) {
@@ -221,7 +256,7 @@ __device__ __forceinline__ void path_coords(const WaveArgs &A, uint32_t slot, ui
         return;
     }
     uint32_t p, s;
-    path_pos_sample(A, A.waveStart + slot, p, s);
+    path_pos_sample(A.ord, A.waveStart + slot, p, s);
     pix = tile_pixel(A, p);
     frame = __ldg(A.sampleOffset) + s;
 }
@@ -257,9 +292,10 @@ __global__ void k_raygen(WaveArgs A) {
         uint32_t q = find_request(A, pid);
         const ReqDev &R = A.reqs[q];
         W = R.width; H = R.height; npix = R.npix;
-        uint64_t local = pid - R.pathStart;
-        pix = tile_pixel_wh(W, H, (uint32_t)(local % npix));
-        frame = R.sampleOffset + (uint32_t)(local / npix);
+        uint32_t p, s;
+        path_pos_sample(R.ord, pid - R.pathStart, p, s);
+        pix = tile_pixel_wh(W, H, p);
+        frame = R.sampleOffset + s;
         A.slotInfo[slot] = make_uint2(pix | (q << 24), frame);
         cp = &R.cam;
     } else {
@@ -1031,7 +1067,7 @@ __device__ __forceinline__ void shade_item(const WaveArgs &A, bool active, uint3
                             cache_record(A.cr, r, hp, -rd, N, m, type, slot);
                             {  // its order key, independent of the path order: sample-major
                                 uint32_t kp, ks;
-                                path_pos_sample(A, A.waveStart + slot, kp, ks);
+                                path_pos_sample(A.ord, A.waveStart + slot, kp, ks);
                                 A.cr[2][r].w = __uint_as_float(
                                     (uint32_t)((uint64_t)ks * A.npix + kp - A.recKeyBase));
                             }
@@ -1425,32 +1461,24 @@ __device__ __forceinline__ void kahan(float &s, float &c, float x) {
     c = (t - s) - y;
     s = t;
 }
-// One thread per pixel position: the wave's samples of the pixel, in sample
+// One thread per pixel position: the paths [first, last) of an order, of which
+// path `first` sits in slot `slot0`; the pixel's samples among them in sample
 // order (path_id), Kahan-added to the film.
-__global__ void k_film(WaveArgs A, float4 *sum, float4 *comp) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= A.npix) return;
-    const uint64_t first = A.waveStart, last = A.waveStart + A.waveCount;
-    // the samples the wave can hold: its first and last paths' samples, widened to their groups
-    uint32_t p0, s0, p1, s1;
-    path_pos_sample(A, first, p0, s0);
-    path_pos_sample(A, last - 1, p1, s1);
-    uint32_t lo, hi;
-    path_group(A, s0, s0, hi);
-    path_group(A, s1, lo, s1);
-    s1 = min(s1, A.spp - 1u);
+__device__ __forceinline__ void film_pixel(const WaveArgs &A, const PathOrder &O, uint64_t first, uint64_t last,
+                                           uint32_t slot0, uint32_t p, uint32_t pix, float4 *sum, float4 *comp) {
+    uint32_t s0, s1;
+    path_samples(O, first, last, s0, s1);
     bool any = false;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = s;
-    const uint32_t pix = tile_pixel(A, p);
     for (uint32_t smp = s0; smp <= s1; smp++) {
-        const uint64_t pid = path_id(A, p, smp);
+        const uint64_t pid = path_id(O, p, smp);
         if (pid < first || pid >= last) continue;
         if (!any) {
             s = sum[pix];
             c = comp[pix];
             any = true;
         }
-        uint32_t slot = (uint32_t)(pid - first);
+        const uint32_t slot = slot0 + (uint32_t)(pid - first);
         float4 le = A.lo_eta[slot];
         float3 L = make_float3(le.x, le.y, le.z);
         if (le.w < 0.0f) {  // NEE of the last bounce pending
@@ -1469,36 +1497,20 @@ __global__ void k_film(WaveArgs A, float4 *sum, float4 *comp) {
         comp[pix] = c;
     }
 }
-
-// Film of request q for the paths of this wave (k_film's order: per pixel,
-// the wave's samples of the request in sample order).
+__global__ void k_film(WaveArgs A, float4 *sum, float4 *comp) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= A.npix) return;
+    film_pixel(A, A.ord, A.waveStart, A.waveStart + A.waveCount, 0u, p, tile_pixel(A, p), sum, comp);
+}
+// Film of request q for its paths in this wave.
 __global__ void k_film_req(WaveArgs A, uint32_t q) {
     const ReqDev &R = A.reqs[q];
     const uint64_t ps = R.pathStart, pe = R.pathStart + (uint64_t)R.npix * R.spp;
     const uint64_t ws = A.waveStart, we = A.waveStart + A.waveCount;
-    const uint64_t lo = (ws > ps ? ws : ps) - ps, hi = (we < pe ? we : pe) - ps;
-    if (hi <= lo) return;
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= min(hi - lo, (uint64_t)R.npix)) return;
-    uint32_t pix = tile_pixel_wh(R.width, R.height, (uint32_t)((lo + t) % R.npix));
-    float4 s = R.sum[pix], c = R.comp[pix];
-    for (uint64_t l = lo + t; l < hi; l += R.npix) {
-        uint32_t slot = (uint32_t)(ps + l - ws);
-        float4 le = A.lo_eta[slot];
-        float3 L = make_float3(le.x, le.y, le.z);
-        if (le.w < 0.0f) {  // NEE of the last bounce pending
-            float4 pa = A.pendA[slot], pe4 = A.pendE[slot];
-            L += make_float3(pa.x, pa.y, pa.z);
-            L += make_float3(pe4.x, pe4.y, pe4.z);
-        }
-        if (isnan(L.x) || isnan(L.y) || isnan(L.z) || isinf(L.x) || isinf(L.y) || isinf(L.z)) L = v3(0.0f);
-        kahan(s.x, c.x, L.x);
-        kahan(s.y, c.y, L.y);
-        kahan(s.z, c.z, L.z);
-        kahan(s.w, c.w, 1.0f);
-    }
-    R.sum[pix] = s;
-    R.comp[pix] = c;
+    const uint64_t lo = ws > ps ? ws : ps, hi = we < pe ? we : pe;
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (hi <= lo || p >= R.npix) return;
+    film_pixel(A, R.ord, lo - ps, hi - ps, (uint32_t)(lo - ws), p, tile_pixel_wh(R.width, R.height, p), R.sum, R.comp);
 }
 
 }  // namespace pt
@@ -1884,14 +1896,9 @@ cudaError_t enqueue_render(const pt_ctx *ctx, Enqueue &E, WaveArgs A, const pt_r
     for (uint64_t ws = 0; ws < total; ws += cap) {
         A.waveStart = ws;
         A.waveCount = (uint32_t)std::min<uint64_t>(cap, total - ws);
-        {  // the samples this wave holds (whole groups of 8): its training records' key range
-            uint32_t p0, s0, p1, s1;
-            path_pos_sample(A, A.waveStart, p0, s0);
-            path_pos_sample(A, A.waveStart + A.waveCount - 1, p1, s1);
-            uint32_t lo, hi;
-            path_group(A, s0, s0, hi);
-            path_group(A, s1, lo, s1);
-            s1 = std::min(s1, A.spp - 1u);
+        {  // the samples this wave holds (whole groups): its training records' key range
+            uint32_t s0, s1;
+            path_samples(A.ord, A.waveStart, A.waveStart + A.waveCount, s0, s1);
             A.recKeyBase = (uint64_t)s0 * A.npix;
             A.recKeyRange = (uint32_t)std::min<uint64_t>((uint64_t)(s1 - s0 + 1) * A.npix, 0xFFFFFFFFull);
         }
@@ -2019,10 +2026,7 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     WaveArgs A;
     A.S = ctx->S;
     A.width = W; A.height = H; A.npix = (uint32_t)npix;
-    A.spp = P->spp;
-    A.spp32 = P->spp & ~31u;  // samples in groups of 32, then of 8 (path_pos_sample)
-    A.spp8 = (P->spp - A.spp32) & ~7u;
-    A.fullTilePix = 32u * (W / 8u) * (H / 4u);
+    A.ord = path_order(W, H, P->spp, !(P->flags & PT_RENDER_RADIANCE_CACHE));
     A.sampleOffset = ctx->d_err + 1;
     A.rngKind = P->rng_kind; A.envMode = P->env_sampling; A.maxDepth = P->max_depth;
     A.cam = P->camera;
@@ -2258,12 +2262,8 @@ cudaError_t enqueue_batch(const pt_ctx *ctx, Enqueue &E, WaveArgs A, const Batch
         A.waveCount = (uint32_t)std::min<uint64_t>(pl.cap, pl.total - A.waveStart);
         chk(enqueue_paths(ctx, E, A, pl.waveDepth[w], G), "paths");
         for (uint32_t j : pl.waveReqs[w]) {
-            const ReqDev &R = hostReqs[j];
-            const uint64_t ps = R.pathStart, pe = ps + (uint64_t)R.npix * R.spp;
-            const uint64_t lo = std::max<uint64_t>(A.waveStart, ps), hi = std::min<uint64_t>(A.waveStart + A.waveCount, pe);
-            const uint64_t cover = std::min<uint64_t>(hi - lo, R.npix);
             E.begin(STG_FILM);
-            k_film_req<<<(unsigned)((cover + kBlock - 1) / kBlock), kBlock, 0, st>>>(A, j);
+            k_film_req<<<(hostReqs[j].npix + kBlock - 1) / kBlock, kBlock, 0, st>>>(A, j);
             E.end();
             chk(cudaGetLastError(), "film launch");
         }
@@ -2369,6 +2369,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         q.pathStart = pl.start[k];
         q.width = P.width; q.height = P.height; q.npix = P.width * P.height; q.spp = P.spp;
         q.sampleOffset = P.sample_offset; q.maxDepth = P.max_depth;
+        q.ord = path_order(P.width, P.height, P.spp, true);
         q.cam = P.camera;
         q.sum = (float4 *)ds;
         q.comp = (float4 *)dc;
@@ -2383,7 +2384,6 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
     memset(&A, 0, sizeof(A));
     A.S = ctx->S;
     A.width = hostReqs[0].width; A.height = hostReqs[0].height; A.npix = hostReqs[0].npix;
-    A.spp = A.spp32 = A.spp8 = A.fullTilePix = 0u;  // batches keep their own path order (slotInfo)
     A.recKeyBase = 0u;
     A.recKeyRange = 0u;
     A.sampleOffset = ctx->d_err + 1;
