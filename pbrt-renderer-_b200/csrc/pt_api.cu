@@ -14,6 +14,184 @@ using namespace pt;
 // ===========================================================================
 namespace pt {
 
+// RGB float32 texels as float4 (alpha 1).
+__global__ void k_env_expand(size_t n, const float *__restrict__ rgb, float4 *env) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        env[i] = make_float4(rgb[3 * i], rgb[3 * i + 1], rgb[3 * i + 2], 1.0f);
+}
+// Indices outside their mesh's vertices raise *bad; one thread per triangle.
+__global__ void k_check_indices(uint32_t n, const uint32_t *__restrict__ meshFirstTri, uint32_t numMeshes,
+                                const pt_material *__restrict__ mats, const uint32_t *__restrict__ idx, uint32_t *bad) {
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n) return;
+    uint32_t a = 0, b = numMeshes;  // last mesh with meshFirstTri <= g
+    while (b - a > 1) {
+        const uint32_t m = (a + b) >> 1;
+        if (meshFirstTri[m] <= g) a = m; else b = m;
+    }
+    const uint32_t base = mats[a].indexOffset + 3u * (g - meshFirstTri[a]), nv = mats[a].vertexCount;
+    if (idx[base] >= nv || idx[base + 1] >= nv || idx[base + 2] >= nv) *bad = 1u;
+}
+
+// ---- envmap tables ------------------------------------------------------------
+// The sums run in the reference's order, element after element, so the bits
+// match; one block per row keeps the row in shared memory, where the serial
+// parts are a chain of additions and not of loads.  Rows beyond kEnvRowMax
+// texels take the one-thread kernels after these.  2048 x 1024 texels: the
+// six kernels 3.5 ms with one thread per row, 0.3 ms so.
+constexpr uint32_t kEnvRowMax = 16384;  // 12 bytes a texel in shared memory
+constexpr int kEnvThreads = 128;
+__device__ __forceinline__ float env_weight(float4 p, float st) {
+    const float l = __fadd_rn(__fadd_rn(__fmul_rn(0.2126f, p.x), __fmul_rn(0.7152f, p.y)), __fmul_rn(0.0722f, p.z));
+    const float w = __fmul_rn(l, st);
+    return w < 0.0f ? 0.0f : w;
+}
+// Conditional CDF row of BuildEnvmapDistribution
+// (src/gpu/DXRApp_Textures.cpp:281-389) and the FP64 weights of the alias
+// tables.
+__global__ void __launch_bounds__(kEnvThreads) k_env_row_block(uint32_t W, const float4 *__restrict__ env,
+                                                               const float *__restrict__ sinRow, float *cond,
+                                                               float *rowSums, double *wall, double *rowSum) {
+    extern __shared__ float sw[];  // weights, then their running sums
+    float *sp = sw + W;
+    __shared__ float total;
+    const uint32_t y = blockIdx.x;
+    const float st = sinRow[y];
+    for (uint32_t x = threadIdx.x; x < W; x += kEnvThreads) {
+        const float w = env_weight(env[(size_t)y * W + x], st);
+        sw[x] = w;
+        wall[(size_t)y * W + x] = (double)w;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float rs = 0.0f;
+#pragma unroll 8
+        for (uint32_t x = 0; x < W; x++) {
+            rs = __fadd_rn(rs, sw[x]);
+            sp[x] = rs;
+        }
+        total = rs;
+        rowSums[y] = rs;
+    } else if (threadIdx.x == 32) {
+        double rs = 0.0;
+#pragma unroll 8
+        for (uint32_t x = 0; x < W; x++) rs = __dadd_rn(rs, (double)sw[x]);
+        rowSum[y] = rs;
+    }
+    __syncthreads();
+    const size_t rb = (size_t)y * (W + 1);
+    const float rs = total;
+    if (rs > 0.0f) {
+        const float inv = __fdiv_rn(1.0f, rs);
+        if (threadIdx.x == 0) cond[rb] = 0.0f;
+        for (uint32_t x = threadIdx.x; x < W; x += kEnvThreads) cond[rb + x + 1] = __fmul_rn(sp[x], inv);
+    } else {
+        for (uint32_t x = threadIdx.x; x <= W; x += kEnvThreads) cond[rb + x] = __fdiv_rn((float)x, (float)W);
+    }
+}
+// Vose alias construction over n weights (FP64) by one block: alias_1d's
+// operations in its order, the weights and the two stacks in shared memory.
+// Returns the weights' sum.
+__device__ double alias_block(const double *w, uint32_t n, float *prob, uint32_t *alias, double *q, uint32_t *stk) {
+    __shared__ double sum;
+    __shared__ uint32_t counts[2];
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) q[i] = w[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+#pragma unroll 8
+        for (uint32_t i = 0; i < n; i++) s = __dadd_rn(s, q[i]);
+        sum = s;
+    }
+    __syncthreads();
+    if (!(sum > 0.0)) {
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) { prob[i] = 1.0f; alias[i] = i; }
+        return sum;
+    }
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) q[i] = __ddiv_rn(__dmul_rn(q[i], (double)n), sum);
+    __syncthreads();
+    if (threadIdx.x < 32) {  // stacks filled in reverse index order, 32 indices at a time
+        uint32_t ns = 0, nl = 0;
+        for (uint32_t k0 = 0; k0 < n; k0 += 32) {
+            const uint32_t k = k0 + threadIdx.x;
+            const bool in = k < n, small = in && q[n - 1 - k] < 1.0;
+            const uint32_t ms = __ballot_sync(0xFFFFFFFFu, small), ml = __ballot_sync(0xFFFFFFFFu, in && !small);
+            const uint32_t below = (1u << threadIdx.x) - 1u;
+            if (small) stk[ns + __popc(ms & below)] = n - 1 - k;
+            else if (in) stk[n - 1 - (nl + __popc(ml & below))] = n - 1 - k;
+            ns += __popc(ms);
+            nl += __popc(ml);
+        }
+        if (threadIdx.x == 0) { counts[0] = ns; counts[1] = nl; }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t ns = counts[0], nl = counts[1];
+        while (ns > 0 && nl > 0) {
+            const uint32_t l = stk[--ns];
+            const uint32_t g = stk[n - 1 - (--nl)];
+            prob[l] = (float)q[l];
+            alias[l] = g;
+            const double r = __dsub_rn(__dadd_rn(q[g], q[l]), 1.0);
+            q[g] = r;
+            if (r < 1.0) stk[ns++] = g;
+            else stk[n - 1 - (nl++)] = g;
+        }
+        while (nl > 0) { const uint32_t g = stk[n - 1 - (--nl)]; prob[g] = 1.0f; alias[g] = g; }
+        while (ns > 0) { const uint32_t l = stk[--ns]; prob[l] = 1.0f; alias[l] = l; }
+    }
+    return sum;
+}
+__global__ void __launch_bounds__(kEnvThreads) k_alias_row_block(uint32_t W, uint32_t H, const double *wall,
+                                                                 const double *rowSum, float *colProb,
+                                                                 uint32_t *colAlias, float *aliasPdf,
+                                                                 const double *total) {
+    extern __shared__ double sq[];
+    const uint32_t y = blockIdx.x;
+    const size_t o = (size_t)y * W;
+    alias_block(wall + o, W, colProb + o, colAlias + o, sq, reinterpret_cast<uint32_t *>(sq + W));
+    const double PI = 3.14159265358979323846, tot = *total, rs = rowSum[y];
+    for (uint32_t x = threadIdx.x; x < W; x += kEnvThreads) {
+        double pp;
+        if (tot > 0.0) pp = rs > 0.0 ? __ddiv_rn(wall[o + x], tot) : 0.0;
+        else pp = __ddiv_rn(1.0, __dmul_rn((double)W, (double)H));
+        aliasPdf[o + x] = (float)__ddiv_rn(__dmul_rn(__dmul_rn(pp, (double)W), (double)H), 2.0 * PI * PI);
+    }
+}
+// The marginal CDF (FP64 running sum over the float row sums), the total of
+// the FP64 row sums and the row alias table; one block.
+__global__ void __launch_bounds__(kEnvThreads) k_env_marginal_block(uint32_t H, const float *__restrict__ rowSums,
+                                                                    const double *rowSum, float *marg, float *rowProb,
+                                                                    uint32_t *rowAlias, double *total) {
+    extern __shared__ double sq[];
+    for (uint32_t y = threadIdx.x; y < H; y += kEnvThreads) sq[y] = (double)rowSums[y];
+    __syncthreads();
+    __shared__ double mt;
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+#pragma unroll 8
+        for (uint32_t y = 0; y < H; y++) t = __dadd_rn(t, sq[y]);
+        mt = t;
+        marg[0] = 0.0f;
+        if (t > 0.0) {
+            const double inv = __ddiv_rn(1.0, t);
+            double acc = 0.0;
+#pragma unroll 8
+            for (uint32_t y = 0; y < H; y++) {
+                acc = __dadd_rn(acc, sq[y]);
+                marg[y + 1] = (float)__dmul_rn(acc, inv);
+            }
+            marg[H] = 1.0f;
+        }
+    }
+    __syncthreads();
+    if (!(mt > 0.0))
+        for (uint32_t y = threadIdx.x; y <= H; y += kEnvThreads) marg[y] = __fdiv_rn((float)y, (float)H);
+    __syncthreads();
+    const double sum = alias_block(rowSum, H, rowProb, rowAlias, sq, reinterpret_cast<uint32_t *>(sq + H));
+    if (threadIdx.x == 0) *total = sum;
+}
+
 // Conditional CDF rows of BuildEnvmapDistribution
 // (src/gpu/DXRApp_Textures.cpp:281-389): one thread per row, sequential
 // float prefix sum in the reference's order, so the bits match.
@@ -302,6 +480,7 @@ int pt_destroy(pt_ctx *ctx) {
     pt_batch_free(ctx);
     pt_branch_free(ctx);
     ctx->free_scene();
+    ctx->sceneMem.release();
     pt_wave_free(ctx);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->d_sobol1) cudaFree(ctx->d_sobol1);
@@ -438,7 +617,8 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         if (pm.indexCount % 3) return ctx->fail(PT_E_INVALID, "indexCount is not a multiple of 3");
         if ((uint64_t)pm.indexOffset + pm.indexCount > d->num_indices) return ctx->fail(PT_E_INVALID, "index range");
         if ((uint64_t)pm.vertexOffset + pm.vertexCount > d->num_vertices) return ctx->fail(PT_E_INVALID, "vertex range");
-        for (uint32_t k = 0; k < pm.indexCount; k++)
+        // emitters' indices are read here (areas below); all meshes' are checked on the device
+        for (uint32_t k = 0; pm.isEmitter && k < pm.indexCount; k++)
             if (d->indices[pm.indexOffset + k] >= pm.vertexCount) return ctx->fail(PT_E_INVALID, "index out of range");
         meshFirstTri[m] = numTris;
         numTris += pm.indexCount / 3;
@@ -469,11 +649,15 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
     std::vector<uint32_t> emitters;
     for (uint32_t m = 0; m < d->num_meshes; m++) {
         pt_material &pm = mats[m];
+        pm.surfaceArea = 0.0f;  // read for emitters only
+        pm.emitterCdfOffset = 0;
+        pm.emitterSelectionProb = 0.0f;
+        if (!pm.isEmitter) continue;
         const uint32_t nt = pm.indexCount / 3;
         std::vector<float> cdf;
-        if (pm.isEmitter) cdf.reserve(nt + 1);
+        cdf.reserve(nt + 1);
         float acc = 0.0f;
-        if (pm.isEmitter) cdf.push_back(0.0f);
+        cdf.push_back(0.0f);
         for (uint32_t t = 0; t < nt; t++) {
             const uint32_t *f = d->indices + pm.indexOffset + 3 * t;
             const float *p0 = d->positions + 3 * (size_t)(pm.vertexOffset + f[0]);
@@ -484,21 +668,17 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
             float cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
             float a = 0.5f * std::sqrt(cx * cx + cy * cy + cz * cz);
             acc = acc + a;
-            if (pm.isEmitter) cdf.push_back(acc);
+            cdf.push_back(acc);
         }
         pm.surfaceArea = acc;
-        pm.emitterCdfOffset = 0;
-        pm.emitterSelectionProb = 0.0f;
-        if (pm.isEmitter) {
-            if (acc > 0.0f) {
-                float inv = 1.0f / acc;
-                for (size_t k = 1; k < cdf.size(); k++) cdf[k] *= inv;
-                cdf.back() = 1.0f;
-            }
-            pm.emitterCdfOffset = (uint32_t)all.size();
-            all.insert(all.end(), cdf.begin(), cdf.end());
-            emitters.push_back(m);
+        if (acc > 0.0f) {
+            float inv = 1.0f / acc;
+            for (size_t k = 1; k < cdf.size(); k++) cdf[k] *= inv;
+            cdf.back() = 1.0f;
         }
+        pm.emitterCdfOffset = (uint32_t)all.size();
+        all.insert(all.end(), cdf.begin(), cdf.end());
+        emitters.push_back(m);
     }
     const uint32_t ne = (uint32_t)emitters.size();
     std::vector<float> pc(ne + 1, 0.0f);
@@ -587,19 +767,21 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
     S.mats = dmats; S.meshClass = dmcls; S.numMeshes = d->num_meshes; S.meshFirstTri = dmft;
     S.emitterCdf = dcdf; S.emitterList = demit; S.emitterCount = ne;
     S.hasGlass = hasGlass ? 1u : 0u;
+    if (numTris) {  // every index within its mesh's vertices, before a kernel follows one
+        uint32_t bad = 0;
+        PT_CUDA(cudaMemsetAsync(ctx->d_err, 0, 4, st));
+        k_check_indices<<<blocks_for(numTris), 256, 0, st>>>(numTris, dmft, S.numMeshes, dmats, didx, ctx->d_err);
+        PT_CUDA(cudaMemcpyAsync(&bad, ctx->d_err, 4, cudaMemcpyDeviceToHost, st));
+        PT_CUDA(cudaMemsetAsync(ctx->d_err, 0, 4, st));
+        PT_CUDA(cudaStreamSynchronize(st));
+        if (bad) return ctx->fail(PT_E_INVALID, "index out of range");
+    }
     // --- BVH ----------------------------------------------------------------------
     if ((rc = pt_build_bvh_device(ctx, dmft, numTris))) return rc;
     // --- envmap -------------------------------------------------------------------
     uint32_t W = d->env_width, H = d->env_height;
-    std::vector<float4> env4;
-    if (!W || !H || !d->env_rgb) {
-        W = H = 1;
-        env4.assign(1, make_float4(0, 0, 0, 1));
-    } else {
-        env4.resize((size_t)W * H);
-        for (size_t i = 0; i < env4.size(); i++)
-            env4[i] = make_float4(d->env_rgb[3 * i], d->env_rgb[3 * i + 1], d->env_rgb[3 * i + 2], 1.0f);
-    }
+    const bool haveEnv = W && H && d->env_rgb;
+    if (!haveEnv) W = H = 1;  // black
     std::vector<float> sinRow(H);
     const float PIf = 3.14159265358979323846f;
     for (uint32_t y = 0; y < H; y++) sinRow[y] = std::sin(PIf * (y + 0.5f) / (float)H);
@@ -620,31 +802,54 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         PT_CUDA(ctx->alloc_scene(&dmguide, kCdfGuide + 1));
         PT_CUDA(ctx->alloc_scene(&dcguide, (size_t)H * (kCdfGuide + 1)));
     }
-    if ((rc = h2d(denv, env4.data(), WH * sizeof(float4)))) return rc;
     {
-        // temporaries: sin table, row sums, FP64 weights, Vose scratch
-        double *wall, *rowSum, *q, *total;
-        uint32_t *stk;
-        cudaError_t e = cudaSuccess;
-        void *tmps[7] = {};
-        e = cudaMalloc(&tmps[0], H * 4 + 16); dsin = (float *)tmps[0];
-        if (e == cudaSuccess) e = cudaMalloc(&tmps[1], H * 4 + 16); drowsum = (float *)tmps[1];
-        if (e == cudaSuccess) e = cudaMalloc(&tmps[2], WH * 8 + 16); wall = (double *)tmps[2];
-        if (e == cudaSuccess) e = cudaMalloc(&tmps[3], H * 8 + 16); rowSum = (double *)tmps[3];
-        if (e == cudaSuccess) e = cudaMalloc(&tmps[4], std::max<size_t>(WH, H) * 8 + 16); q = (double *)tmps[4];
-        if (e == cudaSuccess) e = cudaMalloc(&tmps[5], std::max<size_t>(WH, H) * 4 + 16); stk = (uint32_t *)tmps[5];
-        if (e == cudaSuccess) e = cudaMalloc(&tmps[6], 16); total = (double *)tmps[6];
-        auto freeTmps = [&]() { for (void *p : tmps) if (p) cudaFree(p); };
-        if (e != cudaSuccess) { freeTmps(); return ctx->fail(PT_E_NOMEM, "envmap temporaries"); }
-        cudaMemcpyAsync(dsin, sinRow.data(), H * 4, cudaMemcpyHostToDevice, st);
-        k_env_rows<<<blocks_for(H, 64), 64, 0, st>>>(W, H, denv, dsin, dcond, drowsum);
-        k_env_marginal<<<1, 1, 0, st>>>(H, drowsum, dmarg);
+        // temporaries, one allocation: RGB texels, sin table, row sums, FP64 weights, Vose scratch
+        const bool blocks = W <= kEnvRowMax && H <= kEnvRowMax;
+        const size_t most = std::max<size_t>(WH, H);
+        DeviceArena tmp;
+        float *drgb = nullptr;
+        double *wall, *rowSum, *q = nullptr, *total;
+        uint32_t *stk = nullptr;
+        void *first;
+        cudaError_t e = tmp.alloc(&first, WH * (12 + 8) + (blocks ? 0 : most * 12) + (size_t)H * 16 + 16 + 8 * 256);
+        if (e == cudaSuccess) tmp.chunks[0].used = 0;
+        auto ta = [&](auto **p, size_t bytes) { if (e == cudaSuccess) e = tmp.alloc((void **)p, bytes); };
+        ta(&drgb, WH * 12);
+        ta(&wall, WH * 8);
+        ta(&dsin, (size_t)H * 4);
+        ta(&drowsum, (size_t)H * 4);
+        ta(&rowSum, (size_t)H * 8);
+        ta(&total, 8);
+        if (!blocks) {
+            ta(&q, most * 8);
+            ta(&stk, most * 4);
+        }
+        if (e != cudaSuccess) { tmp.release(); return ctx->fail(PT_E_NOMEM, "envmap temporaries"); }
+        const float black[3] = {0.0f, 0.0f, 0.0f};
+        rc = h2d(drgb, haveEnv ? d->env_rgb : black, WH * 12);
+        if (!rc) rc = h2d(dsin, sinRow.data(), (size_t)H * 4);
+        if (rc) { tmp.release(); return rc; }
+        k_env_expand<<<(unsigned)std::min<size_t>((WH + 255) / 256, 4096), 256, 0, st>>>(WH, drgb, denv);
+        if (blocks) {
+            const size_t mostW = (size_t)W * 12, mostH = (size_t)H * 12;
+            if (mostW > 48 * 1024) cudaFuncSetAttribute(k_alias_row_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mostW);
+            if ((size_t)W * 8 > 48 * 1024) cudaFuncSetAttribute(k_env_row_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W * 8));
+            if (mostH > 48 * 1024) cudaFuncSetAttribute(k_env_marginal_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mostH);
+            k_env_row_block<<<H, kEnvThreads, (size_t)W * 8, st>>>(W, denv, dsin, dcond, drowsum, wall, rowSum);
+            k_env_marginal_block<<<1, kEnvThreads, mostH, st>>>(H, drowsum, rowSum, dmarg, drowProb, drowAlias, total);
+            k_alias_row_block<<<H, kEnvThreads, mostW, st>>>(W, H, wall, rowSum, dcolProb, dcolAlias, dapdf, total);
+        } else {
+            k_env_rows<<<blocks_for(H, 64), 64, 0, st>>>(W, H, denv, dsin, dcond, drowsum);
+            k_env_marginal<<<1, 1, 0, st>>>(H, drowsum, dmarg);
+            k_alias_weights<<<blocks_for(H, 64), 64, 0, st>>>(W, H, denv, dsin, wall, rowSum);
+            k_alias_marginal<<<1, 1, 0, st>>>(H, rowSum, drowProb, drowAlias, q, stk, total);
+            k_alias_rows<<<blocks_for(H, 64), 64, 0, st>>>(W, H, wall, rowSum, dcolProb, dcolAlias, dapdf, q, stk, total);
+        }
         if (dmguide) k_env_guides<<<256, 256, 0, st>>>(W, H, dmarg, dcond, dmguide, dcguide);
-        k_alias_weights<<<blocks_for(H, 64), 64, 0, st>>>(W, H, denv, dsin, wall, rowSum);
-        k_alias_marginal<<<1, 1, 0, st>>>(H, rowSum, drowProb, drowAlias, q, stk, total);
-        k_alias_rows<<<blocks_for(H, 64), 64, 0, st>>>(W, H, wall, rowSum, dcolProb, dcolAlias, dapdf, q, stk, total);
-        e = cudaStreamSynchronize(st);
-        freeTmps();
+        e = cudaGetLastError();
+        const cudaError_t es = cudaStreamSynchronize(st);
+        tmp.release();
+        if (e == cudaSuccess) e = es;
         if (e != cudaSuccess) return ctx->fail(PT_E_CUDA, "envmap tables", cudaGetErrorString(e));
     }
     S.env = denv; S.envW = W; S.envH = H; S.envScale = d->env_scale;
@@ -688,6 +893,7 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         S.vols = dvols; S.dens = ddens; S.maj = dmaj;
     }
     PT_CUDA(cudaStreamSynchronize(st));
+    ctx->sceneMem.trim();
     ctx->clsMask = clsMask;
     ctx->hasScene = true;
     return PT_OK;

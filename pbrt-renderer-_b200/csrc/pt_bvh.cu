@@ -811,17 +811,19 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
     PT_CUDA(ctx->alloc_scene(&codesS, n));
     PT_CUDA(ctx->alloc_scene(&idsS, n));
     PT_CUDA(ctx->alloc_scene(&children, 2 * (size_t)max(n - 1, 1u)));
-    // temporaries
-    std::vector<void *> tmp;
-    auto talloc = [&](void **p, size_t bytes) {
-        cudaError_t e = cudaMalloc(p, bytes + 16);
-        if (e == cudaSuccess) tmp.push_back(*p);
-        return e;
-    };
-    auto cleanup = [&]() { for (void *p : tmp) cudaFree(p); };
+    // temporaries: one allocation, about 230 bytes per triangle and the sort's
+    // tile counts, given back before the build returns
+    DeviceArena tmp;
+    auto cleanup = [&]() { tmp.release(); };
+    {
+        void *all;
+        cudaError_t e = tmp.alloc(&all, (size_t)n * 232 + ((size_t)n / kRsTile + 1) * 1024 + 16384);
+        if (e != cudaSuccess) return ctx->fail(PT_E_NOMEM, "bvh temp", cudaGetErrorString(e));
+        tmp.chunks[0].used = 0;
+    }
 #define TA(p, bytes)                                                                   \
     do {                                                                               \
-        cudaError_t e_ = talloc((void **)&(p), (bytes));                               \
+        cudaError_t e_ = tmp.alloc((void **)&(p), (bytes));                            \
         if (e_ != cudaSuccess) { cleanup(); return ctx->fail(PT_E_NOMEM, "bvh temp", cudaGetErrorString(e_)); } \
     } while (0)
     TA(ids, n * 4);

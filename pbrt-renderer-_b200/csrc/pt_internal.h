@@ -165,6 +165,52 @@ struct BatchState {
     uint64_t tunedSceneGen = 0;
 };
 
+// Device memory handed out by bumping through a few large chunks.  The scene's
+// arena keeps its chunks from one upload to the next (a scene load spent
+// 7 to 47 ms in some 60 cudaMalloc / cudaFree calls); reset() gives all of
+// them back when they hold more than twice what the last scene used, trim()
+// those the new scene does not use, release() everything.
+struct DeviceArena {
+    struct Chunk { char *p; size_t size, used; };
+    std::vector<Chunk> chunks;
+    size_t minChunk;  // 0: chunks of exactly the size asked for (temporaries)
+    explicit DeviceArena(size_t minChunk_ = 0) : minChunk(minChunk_) {}
+    DeviceArena(const DeviceArena &) = delete;
+    DeviceArena &operator=(const DeviceArena &) = delete;
+    ~DeviceArena() { release(); }
+    cudaError_t alloc(void **out, size_t bytes) {
+        bytes = (bytes + 255) & ~(size_t)255;
+        for (Chunk &c : chunks)
+            if (c.size - c.used >= bytes) {
+                *out = c.p + c.used;
+                c.used += bytes;
+                return cudaSuccess;
+            }
+        Chunk c{nullptr, bytes > minChunk ? bytes : minChunk, bytes};
+        const cudaError_t e = cudaMalloc((void **)&c.p, c.size);
+        *out = c.p;
+        if (e == cudaSuccess) chunks.push_back(c);
+        return e;
+    }
+    void reset() {
+        size_t size = 0, used = 0;
+        for (Chunk &c : chunks) { size += c.size; used += c.used; c.used = 0; }
+        if (size > 2 * used + ((size_t)16 << 20)) release();
+    }
+    void trim() {
+        size_t k = 0;
+        for (Chunk &c : chunks) {
+            if (c.used) chunks[k++] = c;
+            else cudaFree(c.p);
+        }
+        chunks.resize(k);
+    }
+    void release() {
+        for (Chunk &c : chunks) cudaFree(c.p);
+        chunks.clear();
+    }
+};
+
 struct pt_ctx {
     int device = 0;
     int numSMs = 148;
@@ -187,7 +233,7 @@ struct pt_ctx {
     cudaEvent_t forkEv[2] = {}, joinEv[2][kBranches] = {};
     bool branchesReady = false;
     std::string err;
-    std::vector<void *> sceneAllocs;  // freed on re-upload / destroy
+    DeviceArena sceneMem{(size_t)1 << 20};  // the uploaded scene's arrays
     pt::DevScene S{};
     bool hasScene = false;
     uint32_t clsMask = 0;  // bit c: shading class c occurs in the scene
@@ -214,14 +260,11 @@ struct pt_ctx {
     }
     template <class T>
     cudaError_t alloc_scene(T **p, size_t count) {
-        cudaError_t e = cudaMalloc((void **)p, count * sizeof(T) + 16);
-        if (e == cudaSuccess) sceneAllocs.push_back((void *)*p);
-        return e;
+        return sceneMem.alloc((void **)p, count * sizeof(T) + 16);
     }
     void free_scene() {
         sceneGen++;
-        for (void *p : sceneAllocs) cudaFree(p);
-        sceneAllocs.clear();
+        sceneMem.reset();
         hasScene = false;
         S = pt::DevScene{};
         d_morton = d_sorted = nullptr;

@@ -18,7 +18,7 @@ def test_one_call_equals_single_samples(w, h, spp, pt, scenes, ctx):
     c = np.zeros((h, w, 4), np.float32)
     for k in range(spp):
         ctx.render(pt.render_params(w, h, 1, cam, max_depth=6, sample_offset=9 + k), s, c)
-    for wave in (0, 5, w * h * 5):
+    for wave in (0, w * h * spp // 37 + 1, w * h * 5):
         s1, c1, st = ctx.render(pt.render_params(w, h, spp, cam, max_depth=6, sample_offset=9, wave_paths=wave))
         assert st.paths == w * h * spp
         assert np.array_equal(s1, s) and np.array_equal(c1, c), wave
