@@ -759,6 +759,7 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         bool homog = d->num_volumes > 0;
         for (uint32_t v = 0; v < d->num_volumes; v++)
             if (d->volumes[v].flags & PT_VOLUME_HETEROGENEOUS) homog = false;
+        ctx->hasHetero = d->num_volumes > 0 && !homog;
         S.mediaWavefront = (homog && !hasSubsurface) ? 1u : 0u;
         S.mediaTrDeferred = 0u;
         if (S.mediaWavefront) clsMask |= 1u << CLS_MEDIUM;

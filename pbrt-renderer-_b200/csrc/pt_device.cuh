@@ -403,73 +403,88 @@ __device__ __forceinline__ uint32_t enumerate_segments(const DevScene &S, float3
     }
     return count;
 }
-__device__ inline bool null_collision(const DevScene &S, uint32_t vi, float3 o, float3 d, float tn, float tf, Rng &rng,
-                               float3 &w, float &ts) {  // Volume.hlsl:236-319
+// One step of the null-collision walk through volume vi (Volume.hlsl:236-319),
+// from t, over the segment ending at tf.
+enum class Walk { kOn, kCollided, kLeft };
+__device__ __forceinline__ Walk null_collision_step(const DevScene &S, uint32_t vi, float3 o, float3 d, float &t,
+                                                    float tf, Rng &rng, float3 &w) {
     const pt_volume &v = S.vols[vi];
     float gmu = vsigma_t_max(v);
     float3 stv = vsigma_t(v);
+    float3 pos = xpos(o, d, t);
+    float lmu, bd;
+    local_majorant(S, vi, pos, d, lmu, bd);
+    if (lmu < 1e-8f) {
+        t += bd;
+        return t >= tf ? Walk::kLeft : Walk::kOn;
+    }
+    float xi = mx(next_float(rng, S.sobol1), 1e-10f);
+    float dt = -logf(xi) / lmu;
+    if (dt > bd) {
+        t += bd;
+        return t >= tf ? Walk::kLeft : Walk::kOn;
+    }
+    t += dt;
+    if (t >= tf) return Walk::kLeft;
+    float dens = vol_density(S, vi, xpos(o, d, t));
+    float pr = sat((dens * gmu) / mx(lmu, 1e-20f));
+    if (pr >= 1.0f - 1e-6f || next_float(rng, S.sobol1) < pr) {
+        w = w * (stv / v3(mx(gmu, 1e-20f)));
+        return Walk::kCollided;
+    }
+    float3 sn = make_float3(__fsub_rn(lmu, __fmul_rn(dens, stv.x)), __fsub_rn(lmu, __fmul_rn(dens, stv.y)),
+                            __fsub_rn(lmu, __fmul_rn(dens, stv.z)));
+    w = w * (sn / v3(mx(lmu * (1.0f - pr), 1e-20f)));
+    return Walk::kOn;
+}
+constexpr uint32_t kWalkSteps = 512;  // per segment
+__device__ inline bool null_collision(const DevScene &S, uint32_t vi, float3 o, float3 d, float tn, float tf, Rng &rng,
+                               float3 &w, float &ts) {
     float t = tn;
-    for (uint32_t step = 0; step < 512; step++) {
-        float3 pos = xpos(o, d, t);
-        float lmu, bd;
-        local_majorant(S, vi, pos, d, lmu, bd);
-        if (lmu < 1e-8f) {
-            t += bd;
-            if (t >= tf) { ts = tf; return false; }
-            continue;
-        }
-        float xi = mx(next_float(rng, S.sobol1), 1e-10f);
-        float dt = -logf(xi) / lmu;
-        if (dt > bd) {
-            t += bd;
-            if (t >= tf) { ts = tf; return false; }
-            continue;
-        }
-        t += dt;
-        if (t >= tf) { ts = tf; return false; }
-        float dens = vol_density(S, vi, xpos(o, d, t));
-        float pr = sat((dens * gmu) / mx(lmu, 1e-20f));
-        if (pr >= 1.0f - 1e-6f || next_float(rng, S.sobol1) < pr) {
-            w = w * (stv / v3(mx(gmu, 1e-20f)));
-            ts = t;
-            return true;
-        }
-        float3 sn = make_float3(__fsub_rn(lmu, __fmul_rn(dens, stv.x)), __fsub_rn(lmu, __fmul_rn(dens, stv.y)),
-                                __fsub_rn(lmu, __fmul_rn(dens, stv.z)));
-        w = w * (sn / v3(mx(lmu * (1.0f - pr), 1e-20f)));
+    for (uint32_t step = 0; step < kWalkSteps; step++) {
+        const Walk r = null_collision_step(S, vi, o, d, t, tf, rng, w);
+        if (r == Walk::kOn) continue;
+        ts = r == Walk::kCollided ? t : tf;
+        return r == Walk::kCollided;
     }
     ts = tf;
     return false;
 }
+// One step of ratio tracking (Volume.hlsl:326-372); kCollided: the
+// transmittance is negligible, `tr` is set to 0.
+__device__ __forceinline__ Walk ratio_step(const DevScene &S, uint32_t vi, float3 o, float3 d, float &t, float tf,
+                                           Rng &rng, float3 &tr) {
+    float3 stv = vsigma_t(S.vols[vi]);
+    float3 pos = xpos(o, d, t);
+    float lmu, bd;
+    local_majorant(S, vi, pos, d, lmu, bd);
+    if (lmu < 1e-8f) {
+        t += bd;
+        return t >= tf ? Walk::kLeft : Walk::kOn;
+    }
+    float xi = mx(next_float(rng, S.sobol1), 1e-10f);
+    float dt = -logf(xi) / lmu;
+    if (dt > bd) {
+        t += bd;
+        return t >= tf ? Walk::kLeft : Walk::kOn;
+    }
+    t += dt;
+    if (t >= tf) return Walk::kLeft;
+    float dens = vol_density(S, vi, xpos(o, d, t));
+    float3 sn = make_float3(__fsub_rn(lmu, __fmul_rn(dens, stv.x)), __fsub_rn(lmu, __fmul_rn(dens, stv.y)),
+                            __fsub_rn(lmu, __fmul_rn(dens, stv.z)));
+    tr = tr * (sn / v3(mx(lmu, 1e-20f)));
+    if (maxc(tr) < 1e-6f) {
+        tr = v3(0.0f);
+        return Walk::kCollided;
+    }
+    return Walk::kOn;
+}
 __device__ inline float3 ratio_tracking(const DevScene &S, uint32_t vi, float3 o, float3 d, float tn, float tf, Rng &rng) {
-    const pt_volume &v = S.vols[vi];  // Volume.hlsl:326-372
-    float3 stv = vsigma_t(v);
     float3 tr = v3(1.0f);
     float t = tn;
-    for (uint32_t step = 0; step < 512; step++) {
-        float3 pos = xpos(o, d, t);
-        float lmu, bd;
-        local_majorant(S, vi, pos, d, lmu, bd);
-        if (lmu < 1e-8f) {
-            t += bd;
-            if (t >= tf) return tr;
-            continue;
-        }
-        float xi = mx(next_float(rng, S.sobol1), 1e-10f);
-        float dt = -logf(xi) / lmu;
-        if (dt > bd) {
-            t += bd;
-            if (t >= tf) return tr;
-            continue;
-        }
-        t += dt;
-        if (t >= tf) return tr;
-        float dens = vol_density(S, vi, xpos(o, d, t));
-        float3 sn = make_float3(__fsub_rn(lmu, __fmul_rn(dens, stv.x)), __fsub_rn(lmu, __fmul_rn(dens, stv.y)),
-                                __fsub_rn(lmu, __fmul_rn(dens, stv.z)));
-        tr = tr * (sn / v3(mx(lmu, 1e-20f)));
-        if (maxc(tr) < 1e-6f) return v3(0.0f);
-    }
+    for (uint32_t step = 0; step < kWalkSteps; step++)
+        if (ratio_step(S, vi, o, d, t, tf, rng, tr) != Walk::kOn) break;
     return tr;
 }
 __device__ inline bool sample_free_flight(const DevScene &S, float3 o, float3 d, float tmax, Rng &rng, float3 &w, float &ts,

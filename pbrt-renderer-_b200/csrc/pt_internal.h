@@ -70,7 +70,8 @@ constexpr int kCounterWords = 32;
 constexpr int kCntShadow = 2, kCntStealExt = 3, kCntClass = 8, kCntStealShadow = kCntClass + CLS_N;
 constexpr int kCntTailRays = 24;  // uint64: extension rays of the tail kernel
 constexpr int kCntRest = 26;      // kernels of the conditional bodies that ran
-static_assert(kCntStealShadow + 1 <= kCntTailRays && kCntRest + 1 <= kCounterWords,
+constexpr int kCntStealFlight = 28, kCntStealRatio = 29;  // (per bounce) claim positions of k_flight / k_ratio
+static_assert(kCntStealShadow + 1 <= kCntTailRays && kCntStealRatio + 1 <= kCounterWords,
               "class queue counts and the tail's ray count must fit the counter block");
 
 // Per-wave buffers of the wavefront integrator (structure of arrays).
@@ -237,6 +238,7 @@ struct pt_ctx {
     pt::DevScene S{};
     bool hasScene = false;
     uint32_t clsMask = 0;  // bit c: shading class c occurs in the scene
+    bool hasHetero = false;  // a heterogeneous medium
     uint32_t numTris = 0;
     uint32_t numWide = 0;
     uint32_t *d_morton = nullptr, *d_sorted = nullptr;

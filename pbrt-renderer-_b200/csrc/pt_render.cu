@@ -100,6 +100,9 @@ struct WaveArgs {
     float4 *so, *sd, *sX, *sthr;
     uint32_t *cntIn, *cntOut, *cntShadow;
     uint32_t *stealExt, *stealShadow;  // next unclaimed queue position of k_extend / k_shadow
+    uint32_t *stealFlight, *stealRatio;  // the same of k_flight / k_ratio
+    uint32_t flightPass;  // free flights in k_flight (heterogeneous media)
+    uint32_t ratioPass;   // NEE ratio tracking in k_ratio
     uint32_t bounce;                   // bounce of the kernels of this launch (uniform over the queue)
     uint32_t *cls, *cntCls;  // shading-class queues (CLS_N x clsStride) and their counts
     uint32_t clsStride;
@@ -331,7 +334,7 @@ __global__ void k_raygen(WaveArgs A) {
     // the first shading pass starts every path from throughput 1 and Lo 0
     // without loading them; they are stored only where something reads them
     // first: the film (no bounce) and the medium free flights of k_extend
-    if (A.S.mediaWavefront || path_depth(A, slot) == 0) {
+    if (A.S.mediaWavefront || A.flightPass || path_depth(A, slot) == 0) {
         A.thr_pdf[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
         A.lo_eta[slot] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
     }
@@ -467,6 +470,21 @@ __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_extend_media(
     extend_queue<true, true>(A);
 }
 
+// The white-noise stream of a deferred NEE ray's ratio tracking, keyed by
+// pixel, sample, bounce and NEE kind (s: the shadow queue entry's slot word).
+__device__ __forceinline__ Rng ratio_rng(const WaveArgs &A, uint32_t s) {
+    const uint32_t slot = s & kShadowSlotMask;
+    Rng r = load_rng(A, slot, make_uint4(0u, 0u, 0u, 0u));  // seeds only
+    Rng t;
+    t.kind = PT_RNG_PCG_HASH;
+    t.pixelSeed = r.pixelSeed;
+    t.sampleIndex = r.sampleIndex;
+    t.dim = 0u;
+    t.white = pcg_hash(r.pixelSeed ^ pcg_hash(r.sampleIndex ^ pcg_hash(((A.rng[slot].z - 1u) << 1) + (s >> 31) +
+                                                                      0x3C6EF372u)));
+    return t;
+}
+
 // ---- shadow: any hit -> pending NEE contribution ---------------------------
 // Shadow queue entry: path slot | kShadowTrLater | kind (0 area, 1 envmap) << 31.
 template <bool MEDIA_TR, class Stack>
@@ -485,19 +503,16 @@ __device__ __forceinline__ void shadow_one(const WaveArgs &A, uint32_t i, Stack 
     float4 X = __ldcs(A.sX + i), Th = __ldcs(A.sthr + i);
     uint32_t s = __ldcs(A.sslot + i);
     const uint32_t slot = s & kShadowSlotMask;
+    if (MEDIA_TR && !occ && (s & kShadowTrLater) && A.ratioPass) {  // left to k_ratio
+        A.sX[i].w = 1.0f;
+        return;
+    }
     if (MEDIA_TR && !occ && (s & kShadowTrLater)) {
         // the ray's medium transmittance (ratio tracking, Volume.hlsl:326-372),
         // estimated only now that the ray is known to be unoccluded: its own
         // white-noise stream, keyed by pixel, sample, bounce and NEE kind.  The
         // shading kernel integrated to the light (area: tmax + 0.001)
-        Rng r = load_rng(A, slot, make_uint4(0u, 0u, 0u, 0u));  // seeds only
-        Rng t;
-        t.kind = PT_RNG_PCG_HASH;
-        t.pixelSeed = r.pixelSeed;
-        t.sampleIndex = r.sampleIndex;
-        t.dim = 0u;
-        t.white = pcg_hash(r.pixelSeed ^ pcg_hash(r.sampleIndex ^ pcg_hash(((A.rng[slot].z - 1u) << 1) + (s >> 31) +
-                                                                          0x3C6EF372u)));
+        Rng t = ratio_rng(A, s);
         const float tm = d.w < 1e19f ? d.w + 0.001f : d.w;
         tr = tr * multi_volume_tr(A.S, make_float3(o.x, o.y, o.z), make_float3(d.x, d.y, d.z), tm, t);
     }
@@ -521,9 +536,191 @@ __device__ __forceinline__ void shadow_queue(const WaveArgs &A) {
         if (i < n) shadow_one<MEDIA_TR>(A, i, K);
     }
 }
+// ---- walks through heterogeneous media ------------------------------------------
+// A walk's length varies from nothing to hundreds of steps within a warp, so
+// one walk per lane to its end leaves 4 to 7 of 32 lanes active.  k_flight
+// (free flights, after the closest-hit kernel) and k_ratio (transmittance of
+// unoccluded NEE rays, after the shadow kernel) advance every lane's walk one
+// step at a time instead, and lanes that are done take the queue's next
+// entries once kWalkRefill of them wait.  Each path's steps and draws are
+// sample_free_flight's and multi_volume_tr's, so the results are too.  Hair in
+// a 128^3 medium, 512 x 512 x 8: 27.5 -> 14.75 ms (15.6 without k_ratio).
+constexpr int kWalkRefill = 8;  // 4: 14.93 ms, 16: 14.91 ms against 14.75 (hair in a medium, 512 x 512 x 8)
+
+// Claims queue positions for the lanes without one (have == false): true with
+// the lane's position in `i`.  All 32 lanes call it; `more` (uniform) is
+// cleared when the queue is exhausted.
+__device__ __forceinline__ bool walk_claim(uint32_t *next, uint32_t n, bool have, bool &more, uint32_t &i) {
+    const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !have);
+    if (!more || (idle != 0xFFFFFFFFu && __popc(idle) < kWalkRefill)) return false;
+    uint32_t base = 0;
+    if (lane_id() == 0) base = atomicAdd(next, (uint32_t)__popc(idle));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    more = base < n && n - base > (uint32_t)__popc(idle);
+    if (have) return false;
+    const uint32_t j = __popc(idle & ((1u << lane_id()) - 1u));
+    if (base >= n || n - base <= j) return false;
+    i = base + j;
+    return true;
+}
+__global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_flight(WaveArgs A) {
+    const DevScene &S = A.S;
+    const uint32_t n = *(volatile uint32_t *)A.cntIn;
+    bool have = false, more = true, inSeg = false;
+    uint32_t i = 0, slot = 0, k = 0, count = 0, step = 0, vi = 0, dim0 = 0, white0 = 0;
+    float t = 0.0f, tf = 0.0f;
+    float3 o = v3(0.0f), d = v3(0.0f), w = v3(1.0f);
+    Rng rng{};
+    Seg segs[8];
+    for (;;) {
+        if (walk_claim(A.stealFlight, n, have, more, i)) {
+            const float4 o4 = A.qoIn[i], d4 = A.qdIn[i], h4 = A.qhit[i];
+            slot = A.bounce == 0u ? i : A.qslotIn[i];
+            rng = load_rng(A, slot, A.rng[slot]);
+            dim0 = rng.dim;
+            white0 = rng.white;
+            o = make_float3(o4.x, o4.y, o4.z);
+            d = make_float3(d4.x, d4.y, d4.z);
+            w = v3(1.0f);
+            count = enumerate_segments(S, o, d, __float_as_uint(h4.y) != 0xFFFFFFFFu ? h4.x : 1e20f, segs);
+            k = 0;
+            inSeg = false;
+            have = true;
+        }
+        if (!__any_sync(0xFFFFFFFFu, have)) {
+            if (more) continue;
+            return;
+        }
+        if (!have) continue;
+        if (!inSeg) {
+            while (k < count && vsigma_t_max(S.vols[segs[k].vi]) < 1e-8f) k++;
+            if (k < count) {
+                vi = segs[k].vi;
+                t = segs[k].tn;
+                tf = segs[k].tf;
+                step = 0;
+                inSeg = true;
+            }
+        }
+        Walk r = Walk::kLeft;
+        if (inSeg) {
+            r = null_collision_step(S, vi, o, d, t, tf, rng, w);
+            if (r == Walk::kOn && ++step == kWalkSteps) r = Walk::kLeft;
+            if (r == Walk::kOn) continue;
+            if (r == Walk::kLeft) {
+                inSeg = false;
+                if (++k < count) continue;
+            }
+        }
+        // the flight is over: collided, or past the last segment.  Only the two
+        // words of the path's state that change are written: the previous
+        // bounce's shadow kernels may be reading the path's bounce beside this
+        if (rng.dim != dim0 || rng.white != white0)
+            *reinterpret_cast<uint2 *>(A.rng + slot) = make_uint2(rng.dim, rng.white);
+        if (w.x != 1.0f || w.y != 1.0f || w.z != 1.0f) {
+            const float4 tp = A.thr_pdf[slot];
+            const float3 t3 = make_float3(tp.x, tp.y, tp.z) * w;
+            A.thr_pdf[slot] = make_float4(t3.x, t3.y, t3.z, tp.w);
+        }
+        if (r == Walk::kCollided) A.qhit[i] = make_float4(t, __uint_as_float(vi | 0x80000000u), 0.0f, 0.0f);
+        have = false;
+    }
+}
+// The shading class of each path after k_flight, in queue order.
+__global__ void __launch_bounds__(kBlock) k_classify(WaveArgs A) {
+    const uint32_t n = *(volatile uint32_t *)A.cntIn;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t gid = __float_as_uint(A.qhit[i].y);
+        const int c = gid == 0xFFFFFFFFu ? (int)CLS_MISS
+                      : (gid >> 31)      ? (int)CLS_MEDIUM
+                                         : (int)__ldg(A.S.meshClass + __ldg(A.S.triMesh + gid));
+        class_append(A, c, i);
+    }
+}
+__global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_ratio(WaveArgs A) {
+    const DevScene &S = A.S;
+    const uint32_t n = min(*(volatile uint32_t *)A.cntShadow, A.shadowCap);
+    bool have = false, more = true, inSeg = false;
+    uint32_t i = 0, s = 0, k = 0, count = 0, step = 0, vi = 0;
+    float t = 0.0f, tf = 0.0f;
+    float3 o = v3(0.0f), d = v3(0.0f), seg = v3(1.0f), tr = v3(1.0f);
+    Rng rng{};
+    Seg segs[8];
+    for (;;) {
+        if (walk_claim(A.stealRatio, n, have, more, i) && A.sX[i].w != 0.0f) {
+            const float4 o4 = A.so[i], d4 = A.sd[i];
+            s = A.sslot[i];
+            rng = ratio_rng(A, s);
+            o = make_float3(o4.x, o4.y, o4.z);
+            d = make_float3(d4.x, d4.y, d4.z);
+            count = enumerate_segments(S, o, d, d4.w < 1e19f ? d4.w + 0.001f : d4.w, segs);
+            tr = v3(1.0f);
+            k = 0;
+            inSeg = false;
+            have = true;
+        }
+        if (!__any_sync(0xFFFFFFFFu, have)) {
+            if (more) continue;
+            return;
+        }
+        if (!have) continue;
+        bool segDone = false;
+        if (!inSeg) {
+            while (k < count && maxc(vsigma_t(S.vols[segs[k].vi])) < 1e-8f) k++;
+            if (k < count) {
+                vi = segs[k].vi;
+                if (S.vols[vi].flags & PT_VOLUME_HETEROGENEOUS) {
+                    t = segs[k].tn;
+                    tf = segs[k].tf;
+                    seg = v3(1.0f);
+                    step = 0;
+                    inSeg = true;
+                } else {
+                    seg = vexp(-vsigma_t(S.vols[vi]) * (segs[k].tf - segs[k].tn));
+                    segDone = true;
+                }
+            }
+        }
+        if (inSeg) {
+            const Walk r = ratio_step(S, vi, o, d, t, tf, rng, seg);
+            if (r == Walk::kOn && ++step < kWalkSteps) continue;
+            inSeg = false;
+            segDone = true;
+        }
+        if (segDone) {
+            tr = tr * seg;
+            if (maxc(tr) < 1e-6f) tr = v3(0.0f);
+            else if (++k < count) continue;
+        }
+        const float4 X = A.sX[i], Th = A.sthr[i];
+        const float3 R = make_float3(Th.x, Th.y, Th.z) * (make_float3(X.x, X.y, X.z) * tr);
+        const float4 out = make_float4(R.x, R.y, R.z, 0.0f);
+        const uint32_t slot = s & kShadowSlotMask;
+        if (s >> 31) __stcs(A.pendE + slot, out);
+        else __stcs(A.pendA + slot, out);
+        have = false;
+    }
+}
 __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_shadow(WaveArgs A) { shadow_queue<false>(A); }
 __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_shadow_media(WaveArgs A) {
     shadow_queue<true>(A);
+}
+
+// The traces and walks of the inline shading form as functions of their own.
+// Inlined at each of its NEE estimates they made a kernel that waited for
+// instructions 9 of 15 cycles per issue (73,728 paths of hair in a medium:
+// shading 3.0 ms inlined, 1.6 ms so).  `S` is the kernel's own parameter
+// (__grid_constant__), so it is passed by address without a copy.
+__device__ __noinline__ bool inline_shadow(const DevScene &S, float3 o, float3 d, float tmin, float tmax, float3 &trans,
+                                           uint32_t *err, uint32_t seed, uint32_t key) {
+    return trace_shadow(S, o, d, tmin, tmax, trans, err, seed, key);
+}
+__device__ __noinline__ float3 inline_tr(const DevScene &S, float3 o, float3 d, float tmax, Rng &rng) {
+    return multi_volume_tr(S, o, d, tmax, rng);
+}
+__device__ __noinline__ bool inline_flight(const DevScene &S, float3 o, float3 d, float tmax, Rng &rng, float3 &w,
+                                           float &ts, uint32_t &svi) {
+    return sample_free_flight(S, o, d, tmax, rng, w, ts, svi);
 }
 
 // One NEE estimate, deferred: either a shadow ray carrying X (everything but
@@ -559,7 +756,7 @@ __device__ __forceinline__ float3 nee_area(const WaveArgs &A, float3 hp, float3 
     float3 trans = v3(1.0f);
     if (INLINE) {
         out.traced = true;
-        if (trace_shadow(S, so, ww, 0.0f, dist - 0.001f, trans, A.err, aseed, alpha_key(bounce, 1u))) return v3(0.0f);
+        if (inline_shadow(S, so, ww, 0.0f, dist - 0.001f, trans, A.err, aseed, alpha_key(bounce, 1u))) return v3(0.0f);
     }
     float3 f;
     float pb;
@@ -567,7 +764,7 @@ __device__ __forceinline__ float3 nee_area(const WaveArgs &A, float3 hp, float3 
     float pe = es.pdfArea * dist * dist / cl;
     float w = balance(pe, pb);
     out.trLater = !INLINE && MEDIA && S.mediaTrDeferred;
-    float3 vt = (INLINE || (MEDIA && S.mediaWavefront && !out.trLater)) ? multi_volume_tr(S, so, ww, dist, rng) : v3(1.0f);
+    float3 vt = INLINE ? inline_tr(S, so, ww, dist, rng) : (MEDIA && S.mediaWavefront && !out.trLater) ? multi_volume_tr(S, so, ww, dist, rng) : v3(1.0f);
     float3 X = es.rad * f * act / v3(mx(pe, 1e-20f)) * w * vt;
     if (INLINE) return X * trans;
     out.ray = true;
@@ -639,14 +836,14 @@ __device__ __forceinline__ float3 nee_ris(const WaveArgs &A, float3 hp, float3 N
     float3 trans = v3(1.0f);
     if (INLINE) {
         out.traced = true;
-        if (trace_shadow(S, so, wiw, 0.0f, dist - 0.001f, trans, A.err, aseed, alpha_key(bounce, 1u))) return v3(0.0f);
+        if (inline_shadow(S, so, wiw, 0.0f, dist - 0.001f, trans, A.err, aseed, alpha_key(bounce, 1u))) return v3(0.0f);
     }
     float3 fu;
     float pdfBsdf;
     material_eval_pdf_t(type, wil, to_local(wiw, T, B, N), m, h, fu, pdfBsdf);
     float wMis = balance(pSA, pdfBsdf);
     out.trLater = !INLINE && MEDIA && S.mediaTrDeferred;
-    float3 vt = (INLINE || (MEDIA && S.mediaWavefront && !out.trLater)) ? multi_volume_tr(S, so, wiw, dist, rng) : v3(1.0f);
+    float3 vt = INLINE ? inline_tr(S, so, wiw, dist, rng) : (MEDIA && S.mediaWavefront && !out.trLater) ? multi_volume_tr(S, so, wiw, dist, rng) : v3(1.0f);
     float3 X = integ * v3(W) * v3(wMis) * vt;
     if (INLINE) return X * trans;
     out.ray = true;
@@ -675,14 +872,14 @@ __device__ __forceinline__ float3 nee_env(const WaveArgs &A, float3 hp, float3 N
     float3 trans = v3(1.0f);
     if (INLINE) {
         out.traced = true;
-        if (trace_shadow(S, so, ww, 0.0f, 1e20f, trans, A.err, aseed, alpha_key(bounce, 2u))) return v3(0.0f);
+        if (inline_shadow(S, so, ww, 0.0f, 1e20f, trans, A.err, aseed, alpha_key(bounce, 2u))) return v3(0.0f);
     }
     float3 f;
     float pb;
     material_eval_pdf_t(type, wil, to_local(ww, T, B, N), m, h, f, pb);
     float w = balance(pe, pb);
     out.trLater = !INLINE && MEDIA && S.mediaTrDeferred;
-    float3 vt = (INLINE || (MEDIA && S.mediaWavefront && !out.trLater)) ? multi_volume_tr(S, so, ww, 1e20f, rng) : v3(1.0f);
+    float3 vt = INLINE ? inline_tr(S, so, ww, 1e20f, rng) : (MEDIA && S.mediaWavefront && !out.trLater) ? multi_volume_tr(S, so, ww, 1e20f, rng) : v3(1.0f);
     float3 X = Le * f * act / v3(mx(pe, 1e-20f)) * w * vt;
     if (INLINE) return X * trans;
     out.ray = true;
@@ -718,13 +915,13 @@ __device__ float3 vol_nee_area(const WaveArgs &A, float3 sp, float3 wo, uint32_t
     if (cl <= 0.0f) return v3(0.0f);
     float3 trans = v3(1.0f);
     if (INLINE) out.traced = true;
-    if (INLINE && trace_shadow(S, sp, wi, 0.001f, dist - 0.001f, trans, A.err, aseed, alpha_key(bounce, 1u)))
+    if (INLINE && inline_shadow(S, sp, wi, 0.001f, dist - 0.001f, trans, A.err, aseed, alpha_key(bounce, 1u)))
         return v3(0.0f);
     float fp = hg(dot(wo, wi), v.phase_g);
     float pe = es.pdfArea * dist * dist / cl;
     float w = balance(pe, fp);
     out.trLater = !INLINE && S.mediaTrDeferred;
-    float3 vt = out.trLater ? v3(1.0f) : multi_volume_tr(S, sp, wi, dist, rng);
+    float3 vt = out.trLater ? v3(1.0f) : INLINE ? inline_tr(S, sp, wi, dist, rng) : multi_volume_tr(S, sp, wi, dist, rng);
     float3 X = es.rad * fp / v3(mx(pe, 1e-20f)) * w * vt;
     if (INLINE) return X * trans;
     out.ray = true;
@@ -746,12 +943,12 @@ __device__ float3 vol_nee_env(const WaveArgs &A, float3 sp, float3 wo, uint32_t 
     if (pe <= 0.0f) return v3(0.0f);
     float3 trans = v3(1.0f);
     if (INLINE) out.traced = true;
-    if (INLINE && trace_shadow(S, sp, wi, 0.001f, 1e20f, trans, A.err, aseed, alpha_key(bounce, 2u)))
+    if (INLINE && inline_shadow(S, sp, wi, 0.001f, 1e20f, trans, A.err, aseed, alpha_key(bounce, 2u)))
         return v3(0.0f);
     float fp = hg(dot(wo, wi), v.phase_g);
     float w = balance(pe, fp);
     out.trLater = !INLINE && S.mediaTrDeferred;
-    float3 vt = out.trLater ? v3(1.0f) : multi_volume_tr(S, sp, wi, 1e20f, rng);
+    float3 vt = out.trLater ? v3(1.0f) : INLINE ? inline_tr(S, sp, wi, 1e20f, rng) : multi_volume_tr(S, sp, wi, 1e20f, rng);
     float3 X = Le * fp / v3(mx(pe, 1e-20f)) * w * vt;
     if (INLINE) return X * trans;
     out.ray = true;
@@ -960,7 +1157,7 @@ __device__ __forceinline__ void shade_item(const WaveArgs &A, bool active, uint3
     if (active) {
         slot = A.bounce == 0u ? i : A.qslotIn[i];
         // bounce 0 outside the medium wavefront: the initial state, known
-        const bool fresh = A.bounce == 0u && !S.mediaWavefront;
+        const bool fresh = A.bounce == 0u && !S.mediaWavefront && !A.flightPass;
         float4 tp = fresh ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : A.thr_pdf[slot];
         float4 le = fresh ? make_float4(0.0f, 0.0f, 0.0f, 1.0f) : A.lo_eta[slot];
         st = A.rng[slot];
@@ -983,11 +1180,17 @@ __device__ __forceinline__ void shade_item(const WaveArgs &A, bool active, uint3
         bool volScat = false;
         if (INLINE && S.numVols > 0) {  // Shaders.hlsl:133-179
             float tSurf = hit ? h4.x : 1e20f;
-            float tsc;
-            uint32_t svi;
-            float3 vw = v3(1.0f);
-            bool sc = sample_free_flight(S, ro, rd, tSurf, rng, vw, tsc, svi);
-            thr *= vw;
+            float tsc = tSurf;
+            uint32_t svi = 0;
+            bool sc = false;
+            if (A.flightPass) {  // k_flight: its weight is in the throughput, a collision in the hit record
+                sc = hit && (gid >> 31);
+                svi = gid & 0x7FFFFFFFu;
+            } else {
+                float3 vw = v3(1.0f);
+                sc = inline_flight(S, ro, rd, tSurf, rng, vw, tsc, svi);
+                thr *= vw;
+            }
             if (sc) {
                 volScat = true;
                 const pt_volume &v = S.vols[svi];
@@ -1305,7 +1508,7 @@ __device__ __forceinline__ void shade_item(const WaveArgs &A, bool active, uint3
     O.thrNee = thrNee;
 }
 template <bool INLINE, int CLS, bool EXTRA = false>
-__global__ void __launch_bounds__(kBlock, ShadeBlocks<CLS>::value) k_shade(WaveArgs A) {
+__global__ void __launch_bounds__(kBlock, ShadeBlocks<CLS>::value) k_shade(const __grid_constant__ WaveArgs A) {
     uint32_t n = CLS == CLS_ANY ? *(volatile uint32_t *)A.cntIn : *(volatile uint32_t *)(A.cntCls + CLS);
     uint32_t iters = (n + gridDim.x * blockDim.x - 1) / (gridDim.x * blockDim.x);
     uint32_t traced = 0;
@@ -1415,7 +1618,7 @@ __device__ __forceinline__ void tail_shade(const WaveArgs &A, Stack &K, uint32_t
     }
 }
 template <bool INLINE>
-__global__ void __launch_bounds__(kBlock, 2) k_tail(WaveArgs A) {
+__global__ void __launch_bounds__(kBlock, 2) k_tail(const __grid_constant__ WaveArgs A) {
     const uint32_t n = *(volatile uint32_t *)A.cntIn;
     if (n > A.tailMax) return;  // uniform: the per-bounce kernels take the rest
     PT_QUEUE_STACK(K)
@@ -1586,7 +1789,7 @@ struct ShadeTable {
 const Kernel *const kShadeCls = ShadeTable<false>::k;
 const Kernel *const kShadeClsX = ShadeTable<true>::k;
 int gExt = 0, gExtC = 0, gExtM = 0, gShadeI = 0, gShadow = 0, gShadowM = 0, gCls[CLS_N], gClsX[CLS_N];
-int gTail = 0, gTailI = 0;
+int gTail = 0, gTailI = 0, gFlight = 0, gRatio = 0;
 
 // STG_CACHE_INFER / STG_CACHE_TRAIN: the cache's network kernels, reported
 // in ms_cache with the rest of the cache's work and on their own in the
@@ -1682,6 +1885,7 @@ struct Grids {
     int ext, extC, extM, shadeI, shadow, shadowM;
     const int *cls, *clsX;
     int tail, tailI;
+    int flight, ratio;
 };
 
 // Launch shape of a kernel that loops over a queue of at most `n` entries of
@@ -1695,8 +1899,9 @@ inline Shape queue_shape(int grid, uint64_t n, uint64_t paths, int numSMs) {
 }
 // Kernels per bounce of a wave (launch counts).
 inline uint32_t bounce_launches(const pt_ctx *ctx, const WaveArgs &A) {
-    if ((ctx->S.numVols > 0 && !A.S.mediaWavefront) || ctx->S.hasSubsurface) return 2;
-    return 2 + (uint32_t)__builtin_popcount(ctx->clsMask | (A.S.mediaWavefront ? 1u << CLS_MEDIUM : 0u));
+    if ((ctx->S.numVols > 0 && !A.S.mediaWavefront) || ctx->S.hasSubsurface) return 2 + A.flightPass;
+    return 2 + (uint32_t)__builtin_popcount(ctx->clsMask | (A.S.mediaWavefront ? 1u << CLS_MEDIUM : 0u)) +
+           2 * A.flightPass + A.ratioPass;
 }
 
 cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t first, uint32_t depth,
@@ -1751,6 +1956,14 @@ bool enqueue_rest_conditional(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32
     return true;
 }
 
+// Which walks through media run in their own kernels: free flights where a
+// medium is heterogeneous, the ratio tracking of deferred NEE rays except in
+// scenes with glass (whose shadow rays carry a transmission of their own).
+void media_passes(const pt_ctx *ctx, WaveArgs &A) {
+    A.flightPass = ctx->hasHetero ? 1u : 0u;
+    A.ratioPass = A.S.mediaTrDeferred && !A.S.hasGlass ? 1u : 0u;
+}
+
 // Raygen and `depth` bounces of one wave (A.waveStart / A.waveCount set).
 // Returns the first failing call's status (cudaSuccess if none).
 cudaError_t enqueue_paths(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t depth, const Grids &G) {
@@ -1792,12 +2005,16 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         A.cntShadow = cnt + kCntShadow;
         A.stealExt = cnt + kCntStealExt;
         A.stealShadow = cnt + kCntStealShadow;
+        A.stealFlight = cnt + kCntStealFlight;
+        A.stealRatio = cnt + kCntStealRatio;
         A.cntCls = cnt + kCntClass;
         auto shape = [&](int grid, uint64_t n) { return queue_shape(grid, n, A.waveCount, ctx->numSMs); };
         if (tail && b == tail_bounce(depth, A, ctx->dbgTail)) {  // the remaining bounces of every path in one launch, when few are left
             joinShadow();
             E.begin(STG_TAIL);
-            if (inl) k_tail<true><<<G.tailI, kBlock, 0, st>>>(A);
+            WaveArgs T = A;  // a path's flights run in its own thread
+            T.flightPass = 0u;
+            if (inl) k_tail<true><<<G.tailI, kBlock, 0, st>>>(T);
             else k_tail<false><<<G.tail, kBlock, 0, st>>>(A);
             if (fj) {
                 if (enqueue_rest_conditional(ctx, E, A, b, depth, G, err)) return err;
@@ -1816,13 +2033,28 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
             E.begin(STG_EXTEND);
             k_extend<false><<<x.grid, x.block, 0, st>>>(A);
             E.end();
+            if (A.flightPass) {
+                const Shape f = shape(G.flight, A.waveCount);
+                E.begin(STG_EXTEND);
+                k_flight<<<f.grid, f.block, 0, st>>>(A);
+                E.end();
+            }
             E.begin(STG_SHADE);
             k_shade<true, CLS_ANY><<<h.grid, h.block, 0, st>>>(A);
             E.end();
             continue;
         }
         E.begin(STG_EXTEND);
-        if (A.S.mediaWavefront) {
+        if (A.flightPass) {
+            const Shape x = shape(G.ext, A.waveCount), f = shape(G.flight, A.waveCount);
+            k_extend<false><<<x.grid, x.block, 0, st>>>(A);
+            E.end();
+            E.begin(STG_EXTEND);
+            k_flight<<<f.grid, f.block, 0, st>>>(A);
+            E.end();
+            E.begin(STG_EXTEND);
+            k_classify<<<x.grid, x.block, 0, st>>>(A);
+        } else if (A.S.mediaWavefront) {
             const Shape x = shape(G.extM, A.waveCount);
             k_extend_media<<<x.grid, x.block, 0, st>>>(A);
         } else {
@@ -1867,6 +2099,12 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         if (A.S.mediaTrDeferred) k_shadow_media<<<w.grid, w.block, 0, ss>>>(A);
         else k_shadow<<<w.grid, w.block, 0, ss>>>(A);
         E.end();
+        if (A.ratioPass) {
+            const Shape q = shape(G.ratio, 2ull * A.waveCount);
+            E.begin(STG_SHADOW);
+            k_ratio<<<q.grid, q.block, 0, ss>>>(A);
+            E.end();
+        }
         if (fj) {
             chk(cudaEventRecord(fj->joinEv[0], ss));
             shadowOpen = true;
@@ -1886,7 +2124,7 @@ cudaError_t enqueue_render(const pt_ctx *ctx, Enqueue &E, WaveArgs A, const pt_r
         if (err == cudaSuccess && e != cudaSuccess) err = e;
     };
     const bool cached = A.cacheOn != 0;
-    const Grids G{gExt, gExtC, gExtM, gShadeI, gShadow, gShadowM, gCls, gClsX, gTail, gTailI};
+    const Grids G{gExt, gExtC, gExtM, gShadeI, gShadow, gShadowM, gCls, gClsX, gTail, gTailI, gFlight, gRatio};
     chk(cudaMemsetAsync(B.counters, 0, kCounterWords * sizeof(uint32_t), st));
     chk(cudaMemsetAsync(ctx->d_err, 0, 4, st));
     if (cached) {  // per-call cache counters: records [2], queries of the call [5], records with targets [6]
@@ -2022,6 +2260,8 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
         }
         gTail = grid_for(ctx, (const void *)k_tail<false>);
         gTailI = grid_for(ctx, (const void *)k_tail<true>);
+        gFlight = grid_for(ctx, (const void *)k_flight);
+        gRatio = grid_for(ctx, (const void *)k_ratio);
     }
     WaveArgs A;
     A.S = ctx->S;
@@ -2048,6 +2288,7 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
         A.S.mediaWavefront = 1u;  // heterogeneous media (homogeneous-only scenes have it already)
         A.S.mediaTrDeferred = 1u;
     }
+    media_passes(ctx, A);
     A.cacheOn = (P->flags & PT_RENDER_RADIANCE_CACHE) ? 1u : 0u;
     A.trainOn = A.unbiasedEvery = A.recCap = A.queryCap = 0;
     A.roughThr = 0.0f;
@@ -2322,6 +2563,8 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         }
         gTail = grid_for(ctx, (const void *)k_tail<false>);
         gTailI = grid_for(ctx, (const void *)k_tail<true>);
+        gFlight = grid_for(ctx, (const void *)k_flight);
+        gRatio = grid_for(ctx, (const void *)k_ratio);
     }
     if (gridScale <= 0.0f) gridScale = (Bt.tunedWave && Bt.tunedSceneGen == ctx->sceneGen) ? Bt.tunedGrid : 1.0f;
     auto sc = [&](int g) { return std::max(ctx->numSMs, (int)((float)g * gridScale)); };
@@ -2331,7 +2574,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         clsGX[c] = sc(gClsX[c]);
     }
     const Grids G{sc(gExt), sc(gExtC), sc(gExtM), sc(gShadeI), sc(gShadow), sc(gShadowM), clsG, clsGX, sc(gTail),
-                  sc(gTailI)};
+                  sc(gTailI), sc(gFlight), sc(gRatio)};
 
     const BatchPlan pl = batch_plan(R, n, cap);
     // films: the callers' device films, device copies of host films, or the tuning scratch
@@ -2406,6 +2649,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         A.S.mediaWavefront = 1u;  // heterogeneous media (homogeneous-only scenes have it already)
         A.S.mediaTrDeferred = 1u;
     }
+    media_passes(ctx, A);
     // the launch graph depends on the batch's shape, not on cameras, offsets or films (device table)
     std::vector<uint64_t> key = {n, pl.cap, R[0].params.rng_kind, R[0].params.env_sampling, R[0].params.flags,
                                  ctx->sceneGen,
