@@ -19,9 +19,11 @@ __global__ void k_env_expand(size_t n, const float *__restrict__ rgb, float4 *en
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         env[i] = make_float4(rgb[3 * i], rgb[3 * i + 1], rgb[3 * i + 2], 1.0f);
 }
-// Indices outside their mesh's vertices raise *bad; one thread per triangle.
-__global__ void k_check_indices(uint32_t n, const uint32_t *__restrict__ meshFirstTri, uint32_t numMeshes,
-                                const pt_material *__restrict__ mats, const uint32_t *__restrict__ idx, uint32_t *bad) {
+// Shading records of each triangle (vertices and mesh, class); indices outside
+// their mesh's vertices raise *bad.
+__global__ void k_tri_records(uint32_t n, const uint32_t *__restrict__ meshFirstTri, uint32_t numMeshes,
+                              const pt_material *__restrict__ mats, const uint32_t *__restrict__ meshClass,
+                              const uint32_t *__restrict__ idx, uint4 *triIdx, uint8_t *triClass, uint32_t *bad) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     uint32_t a = 0, b = numMeshes;  // last mesh with meshFirstTri <= g
@@ -29,8 +31,19 @@ __global__ void k_check_indices(uint32_t n, const uint32_t *__restrict__ meshFir
         const uint32_t m = (a + b) >> 1;
         if (meshFirstTri[m] <= g) a = m; else b = m;
     }
-    const uint32_t base = mats[a].indexOffset + 3u * (g - meshFirstTri[a]), nv = mats[a].vertexCount;
-    if (idx[base] >= nv || idx[base + 1] >= nv || idx[base + 2] >= nv) *bad = 1u;
+    const pt_material &m = mats[a];
+    const uint32_t base = m.indexOffset + 3u * (g - meshFirstTri[a]), nv = m.vertexCount;
+    const uint32_t i0 = idx[base], i1 = idx[base + 1], i2 = idx[base + 2];
+    if (i0 >= nv || i1 >= nv || i2 >= nv) *bad = 1u;
+    triIdx[g] = make_uint4(m.vertexOffset + i0, m.vertexOffset + i1, m.vertexOffset + i2, a);
+    triClass[g] = (uint8_t)meshClass[a];
+}
+__global__ void k_pack_vertices(size_t n, const float *__restrict__ pos, const float *__restrict__ nrm, float4 *pos4,
+                                float4 *nrm4) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        pos4[i] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], 0.0f);
+        nrm4[i] = make_float4(nrm[3 * i], nrm[3 * i + 1], nrm[3 * i + 2], 0.0f);
+    }
 }
 
 // ---- envmap tables ------------------------------------------------------------
@@ -426,6 +439,38 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSm) k_trace_shadow
     tr[3 * i] = t.x; tr[3 * i + 1] = t.y; tr[3 * i + 2] = t.z;
 }
 
+// The same with 8 lanes per ray, for queries that fit the GPU at once so
+// (kTraceCoopMax); occlusion only without glass.
+constexpr size_t kTraceCoopMax = 148u * 32u * 4u;
+__global__ void __launch_bounds__(kTraceBlock) k_trace_closest8(DevScene S, const float *rays, size_t n, pt_hit *out,
+                                                                uint32_t *err) {
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    if (i >= n) return;
+    const Group8 G = group8();
+    const float *r = rays + 8 * i;
+    const Hit h = trace_closest8(G, S, make_float3(r[0], r[1], r[2]), make_float3(r[4], r[5], r[6]), r[3], r[7], err,
+                                 (uint32_t)i, 0u);
+    if (G.j) return;
+    if (h.gid != 0xFFFFFFFFu) {
+        const uint32_t m = S.triMesh[h.gid];
+        out[i] = pt_hit{h.t, m, h.gid - S.meshFirstTri[m], h.u, h.v, 1u};
+    } else {
+        out[i] = pt_hit{0.0f, 0u, 0u, 0.0f, 0.0f, 0u};
+    }
+}
+__global__ void __launch_bounds__(kTraceBlock) k_trace_shadow8(DevScene S, const float *rays, size_t n, uint32_t *occ,
+                                                               float *tr, uint32_t *err) {
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    if (i >= n) return;
+    const Group8 G = group8();
+    const float *r = rays + 8 * i;
+    const bool o = trace_shadow8(G, S, make_float3(r[0], r[1], r[2]), make_float3(r[4], r[5], r[6]), r[3], r[7], err,
+                                 (uint32_t)i, 0u);
+    if (G.j) return;
+    occ[i] = o ? 1u : 0u;
+    tr[3 * i] = tr[3 * i + 1] = tr[3 * i + 2] = 1.0f;
+}
+
 }  // namespace pt
 
 // ===========================================================================
@@ -764,14 +809,24 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         S.mediaTrDeferred = 0u;
         if (S.mediaWavefront) clsMask |= 1u << CLS_MEDIUM;
     }
-    S.pos = dpos; S.nrm = dnrm; S.uv = duv; S.tan = dtan; S.idx = didx;
-    S.mats = dmats; S.meshClass = dmcls; S.numMeshes = d->num_meshes; S.meshFirstTri = dmft;
+    S.pos = dpos; S.uv = duv; S.tan = dtan; S.idx = didx;
+    S.mats = dmats; S.numMeshes = d->num_meshes; S.meshFirstTri = dmft;
     S.emitterCdf = dcdf; S.emitterList = demit; S.emitterCount = ne;
     S.hasGlass = hasGlass ? 1u : 0u;
+    float4 *dpos4, *dnrm4;
+    uint4 *dtidx;
+    uint8_t *dtcls;
+    PT_CUDA(ctx->alloc_scene(&dpos4, nv + 1));
+    PT_CUDA(ctx->alloc_scene(&dnrm4, nv + 1));
+    PT_CUDA(ctx->alloc_scene(&dtidx, (size_t)numTris + 1));
+    PT_CUDA(ctx->alloc_scene(&dtcls, (size_t)numTris + 1));
+    S.pos4 = dpos4; S.nrm4 = dnrm4; S.triIdx = dtidx; S.triClass = dtcls;
+    if (nv) k_pack_vertices<<<(unsigned)std::min<size_t>((nv + 255) / 256, 4096), 256, 0, st>>>(nv, dpos, dnrm, dpos4, dnrm4);
     if (numTris) {  // every index within its mesh's vertices, before a kernel follows one
         uint32_t bad = 0;
         PT_CUDA(cudaMemsetAsync(ctx->d_err, 0, 4, st));
-        k_check_indices<<<blocks_for(numTris), 256, 0, st>>>(numTris, dmft, S.numMeshes, dmats, didx, ctx->d_err);
+        k_tri_records<<<blocks_for(numTris), 256, 0, st>>>(numTris, dmft, S.numMeshes, dmats, dmcls, didx, dtidx, dtcls,
+                                                           ctx->d_err);
         PT_CUDA(cudaMemcpyAsync(&bad, ctx->d_err, 4, cudaMemcpyDeviceToHost, st));
         PT_CUDA(cudaMemsetAsync(ctx->d_err, 0, 4, st));
         PT_CUDA(cudaStreamSynchronize(st));
@@ -1184,7 +1239,11 @@ int pt_trace_closest(pt_ctx *ctx, const float *rays, size_t n, pt_hit *out, uint
     int rc = s.setup();
     if (rc) return rc;
     cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
-    k_trace_closest<<<blocks_for(n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (pt_hit *)s.dev(1),
+    if (n <= kTraceCoopMax)
+        k_trace_closest8<<<blocks_for(8 * n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n,
+                                                                                     (pt_hit *)s.dev(1), ctx->d_err);
+    else
+        k_trace_closest<<<blocks_for(n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (pt_hit *)s.dev(1),
                                                              ctx->d_err);
     rc = s.finish();
     if (rc) return rc;
@@ -1206,7 +1265,11 @@ int pt_trace_shadow(pt_ctx *ctx, const float *rays, size_t n, uint32_t *occ, flo
     int rc = s.setup();
     if (rc) return rc;
     cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
-    k_trace_shadow<<<blocks_for(n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (uint32_t *)s.dev(1),
+    if (n <= kTraceCoopMax && !ctx->S.hasGlass)
+        k_trace_shadow8<<<blocks_for(8 * n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(
+            ctx->S, (float *)s.dev(0), n, (uint32_t *)s.dev(1), (float *)s.dev(2), ctx->d_err);
+    else
+        k_trace_shadow<<<blocks_for(n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n, (uint32_t *)s.dev(1),
                                                             (float *)s.dev(2), ctx->d_err);
     rc = s.finish();
     if (rc) return rc;

@@ -43,11 +43,18 @@ struct DevScene {
     const uint32_t *triMesh;      // global triangle id -> mesh
     const uint32_t *meshFirstTri; // mesh -> first global triangle id
     const pt_material *mats;
-    const uint32_t *meshClass;    // mesh -> shading class of its hits
     uint32_t numMeshes;
     uint32_t hasGlass;            // any mirror/dielectric mesh (non-opaque for shadow rays)
-    const float *pos, *nrm, *uv, *tan;
+    const float *pos, *uv, *tan;
     const uint32_t *idx;
+    // for shading: vertex positions and normals as 16-byte records, and per
+    // global triangle id its three vertices and mesh in one, and its shading
+    // class.  One load leads from a hit to its vertices; through triMesh, the
+    // mesh's first triangle, its material's offsets and the indices it was
+    // four dependent ones and 18 scalar vertex loads after them
+    const float4 *pos4, *nrm4;
+    const uint4 *triIdx;
+    const uint8_t *triClass;
     // emitters (src/gpu/DXRApp_Scene.cpp:243-299)
     const float *emitterCdf;
     const uint32_t *emitterList;
@@ -114,6 +121,21 @@ __device__ __forceinline__ float next_float(Rng &r, const uint32_t *__restrict__
 __device__ __forceinline__ float3 ld3(const float *b, uint32_t i) {
     return make_float3(__ldg(b + 3 * i), __ldg(b + 3 * i + 1), __ldg(b + 3 * i + 2));
 }
+__device__ __forceinline__ float3 ld4(const float4 *b, uint32_t i) {
+    const float4 v = __ldg(b + i);
+    return make_float3(v.x, v.y, v.z);
+}
+// Material of mesh `mesh` by 16-byte loads (144 bytes; the array is aligned).
+__device__ __forceinline__ pt_material load_material(const DevScene &S, uint32_t mesh) {
+    struct alignas(16) Quads { uint4 q[9]; } w;
+    static_assert(sizeof(Quads) == sizeof(pt_material), "material record");
+    const uint4 *src = reinterpret_cast<const uint4 *>(S.mats + mesh);
+#pragma unroll
+    for (int k = 0; k < 9; k++) w.q[k] = __ldg(src + k);
+    pt_material m;
+    memcpy(&m, &w, sizeof(m));
+    return m;
+}
 __device__ __forceinline__ void tri_vidx(const DevScene &S, uint32_t mesh, uint32_t prim, uint32_t &i0, uint32_t &i1,
                                          uint32_t &i2) {
     const pt_material &m = S.mats[mesh];
@@ -121,10 +143,6 @@ __device__ __forceinline__ void tri_vidx(const DevScene &S, uint32_t mesh, uint3
     i0 = m.vertexOffset + __ldg(S.idx + base);
     i1 = m.vertexOffset + __ldg(S.idx + base + 1);
     i2 = m.vertexOffset + __ldg(S.idx + base + 2);
-}
-__device__ __forceinline__ float3 geometric_normal(const DevScene &S, uint32_t i0, uint32_t i1, uint32_t i2) {
-    float3 p0 = ld3(S.pos, i0), p1 = ld3(S.pos, i1), p2 = ld3(S.pos, i2);
-    return normalize(cross(p1 - p0, p2 - p0));
 }
 
 // ---------------------------------------------------------------------------
@@ -285,7 +303,7 @@ __device__ __forceinline__ EmitterSample sample_emitter(const DevScene &S, Rng &
     uint32_t tri = min(cdf_search(S.emitterCdf + m.emitterCdfOffset, nt + 1, u), nt - 1);
     uint32_t i0, i1, i2;
     tri_vidx(S, id, tri, i0, i1, i2);
-    float3 p0 = ld3(S.pos, i0), p1 = ld3(S.pos, i1), p2 = ld3(S.pos, i2);
+    float3 p0 = ld4(S.pos4, i0), p1 = ld4(S.pos4, i1), p2 = ld4(S.pos4, i2);
     float r1 = next_float(rng, S.sobol1), r2 = next_float(rng, S.sobol1);
     float sr1 = sqrtf(r1);
     es.pos = (1.0f - sr1) * p0 + sr1 * (1.0f - r2) * p1 + sr1 * r2 * p2;
@@ -567,11 +585,9 @@ __device__ __forceinline__ float4 tex_sample(const DevScene &S, uint32_t index, 
 // ComputeUVFootprint (shaders/GeometryUtils.hlsli:120-145): world-space pixel
 // footprint at distance hitT mapped to UV space by the triangle's UV/world
 // area ratio.
-__device__ __forceinline__ float uv_footprint(const DevScene &S, uint32_t mesh, uint32_t prim, float hitT,
+__device__ __forceinline__ float uv_footprint(const DevScene &S, uint32_t i0, uint32_t i1, uint32_t i2, float hitT,
                                               uint32_t width, uint32_t height) {
-    uint32_t i0, i1, i2;
-    tri_vidx(S, mesh, prim, i0, i1, i2);
-    float3 p0 = ld3(S.pos, i0), p1 = ld3(S.pos, i1), p2 = ld3(S.pos, i2);
+    float3 p0 = ld4(S.pos4, i0), p1 = ld4(S.pos4, i1), p2 = ld4(S.pos4, i2);
     float u0 = __ldg(S.uv + 2 * i0), v0 = __ldg(S.uv + 2 * i0 + 1);
     float u1 = __ldg(S.uv + 2 * i1), v1 = __ldg(S.uv + 2 * i1 + 1);
     float u2 = __ldg(S.uv + 2 * i2), v2 = __ldg(S.uv + 2 * i2 + 1);
@@ -604,12 +620,9 @@ __device__ __forceinline__ float2 interp_uv(const DevScene &S, uint32_t i0, uint
 // traversal meets the candidates.
 __device__ __forceinline__ bool alpha_pass(const DevScene &S, uint32_t gid, float b1, float b2, uint32_t seed,
                                            uint32_t key, bool shadow) {
-    uint32_t mesh = __ldg(S.triMesh + gid);
-    uint32_t prim = gid - __ldg(S.meshFirstTri + mesh);
-    uint32_t i0, i1, i2;
-    tri_vidx(S, mesh, prim, i0, i1, i2);
-    float2 uv = interp_uv(S, i0, i1, i2, b1, b2);
-    float4 c = tex_sample(S, __ldg(&S.mats[mesh].alphaTexIndex), uv.x, uv.y, 0.0f);
+    const uint4 ti = __ldg(S.triIdx + gid);
+    float2 uv = interp_uv(S, ti.x, ti.y, ti.z, b1, b2);
+    float4 c = tex_sample(S, __ldg(&S.mats[ti.w].alphaTexIndex), uv.x, uv.y, 0.0f);
     float a = shadow ? (c.w < 1.0f ? c.w : c.x) : c.x;
     if (a < 0.01f) return false;
     float xi = u32_to_unit(pcg_hash(seed ^ pcg_hash(key * 0x9e3779b9u ^ gid)));
@@ -960,6 +973,141 @@ __device__ __forceinline__ bool trace_shadow(const DevScene &S, float3 o, float3
                                              float3 &trans, uint32_t *err, uint32_t seed = 0u, uint32_t key = 0u) {
     TravStack K;
     return trace_shadow_on(K, S, o, d, tmin, tmax, trans, err, seed, key);
+}
+
+// ---------------------------------------------------------------------------
+// traversal by 8 lanes per ray
+// ---------------------------------------------------------------------------
+// For queues too short to fill the GPU, where a kernel lasts as long as its
+// slowest ray: the 8 lanes of a group test a node's 8 children at once (lane
+// j the slot j ^ oct, so a ballot gives the hits in visit order) and a node's
+// triangles 8 at a time; everything else is the same in all lanes.  Boxes,
+// their order and each triangle's arithmetic are the one-lane form's, so the
+// results are its bits.  All 8 lanes of a group call these together.
+struct Group8 {
+    uint32_t mask, shift, j;
+};
+__device__ __forceinline__ Group8 group8() {
+    const uint32_t lane = threadIdx.x & 31u;
+    return {0xFFu << (lane & 24u), lane & 24u, lane & 7u};
+}
+// Children of node `ni`: hits of internal children (visit order) and the
+// triangle mask, equal in all lanes.
+__device__ __forceinline__ void intersect_node8(const Group8 &G, const DevScene &S, uint32_t ni, const RayPre &r,
+                                                float tmin, float tmax, uint32_t &gBase, uint32_t &gImask,
+                                                uint32_t &gHits, uint32_t &tBase, uint32_t &tHits) {
+    const uint8_t *nb = reinterpret_cast<const uint8_t *>(S.nodes + ni);
+    const uint32_t slot = G.j ^ r.oct;
+    const uint4 n0 = __ldg(reinterpret_cast<const uint4 *>(nb));
+    const uint2 n1 = __ldg(reinterpret_cast<const uint2 *>(nb + 16));
+    const uint32_t meta = __ldg(nb + 24 + slot);
+    float lx = (float)__ldg(nb + 32 + slot), ly = (float)__ldg(nb + 40 + slot), lz = (float)__ldg(nb + 48 + slot);
+    float hx = (float)__ldg(nb + 56 + slot), hy = (float)__ldg(nb + 64 + slot), hz = (float)__ldg(nb + 72 + slot);
+    if (r.idir.x < 0.0f) { const float t = lx; lx = hx; hx = t; }
+    if (r.idir.y < 0.0f) { const float t = ly; ly = hy; hy = t; }
+    if (r.idir.z < 0.0f) { const float t = lz; lz = hz; hz = t; }
+    const float sx = __uint_as_float((n0.w & 0xFFu) << 23) * r.idir.x;
+    const float sy = __uint_as_float(((n0.w >> 8) & 0xFFu) << 23) * r.idir.y;
+    const float sz = __uint_as_float(((n0.w >> 16) & 0xFFu) << 23) * r.idir.z;
+    const float ox = (__uint_as_float(n0.x) - r.o.x) * r.idir.x, oy = (__uint_as_float(n0.y) - r.o.y) * r.idir.y,
+                oz = (__uint_as_float(n0.z) - r.o.z) * r.idir.z;
+    const float t0 = fmax3(fmaf(lx, sx, ox), fmaf(ly, sy, oy), fmaxf(fmaf(lz, sz, oz), tmin));
+    const float t1 = fmin3(fmaf(hx, sx, ox), fmaf(hy, sy, oy), fminf(fmaf(hz, sz, oz), tmax));
+    const bool hit = t0 <= __fmul_rn(t1, 1.00000024f);
+    gImask = n0.w >> 24;
+    const bool internal = (gImask >> slot) & 1u;
+    gHits = (__ballot_sync(G.mask, hit && internal) >> G.shift) & 0xFFu;
+    tHits = __reduce_or_sync(G.mask, hit && !internal ? (meta >> 5) << (meta & 31u) : 0u);
+    gBase = n1.x;
+    tBase = n1.y;
+}
+// The next node to visit (false: none left, or an error, flagged in *err).
+__device__ __forceinline__ bool next_node8(const DevScene &S, TravStack &K, const RayPre &r, uint32_t &gBase,
+                                           uint32_t &gImask, uint32_t &gHits, int &sp, uint32_t &visits,
+                                           uint32_t &child, uint32_t *err) {
+    if (gHits == 0) {
+        if (sp == 0) return false;
+        const uint2 e = K.get(--sp);
+        gBase = e.x;
+        gImask = e.y >> 8;
+        gHits = e.y & 0xFFu;
+    }
+    const uint32_t slot = (uint32_t)(__ffs(gHits) - 1) ^ r.oct;
+    gHits &= gHits - 1;
+    child = gBase + __popc(gImask & ((1u << slot) - 1u));
+    if (++visits > S.numNodes || child >= S.numNodes) {
+        if (err) atomicOr(err, 4u);
+        return false;
+    }
+    if (gHits) {
+        if (sp == kTraversalStack) {
+            if (err) atomicOr(err, 1u);
+            return false;
+        }
+        K.put(sp++, gBase, (gImask << 8) | gHits);
+    }
+    return true;
+}
+__device__ __forceinline__ Hit trace_closest8(const Group8 &G, const DevScene &S, float3 o, float3 d, float tmin,
+                                              float tmax, uint32_t *err, uint32_t seed, uint32_t key) {
+    Hit h;
+    h.t = tmax; h.u = 0.0f; h.v = 0.0f; h.gid = 0xFFFFFFFFu;
+    if (S.numNodes == 0) return h;
+    TravStack K;
+    const RayPre r = ray_pre(o, d);
+    uint32_t gBase, gImask, gHits, tBase, tHits, visits = 1, child = 0;
+    int sp = 0;
+    do {
+        intersect_node8(G, S, child, r, tmin, h.t, gBase, gImask, gHits, tBase, tHits);
+        for (uint32_t k = 0; tHits >> (8u * k); k++) {
+            float t = 0.0f, u = 0.0f, v = 0.0f;
+            uint32_t g = 0xFFFFFFFFu;
+            bool ok = (tHits >> (8u * k + G.j)) & 1u;
+            if (ok) {
+                const float4 *tp = S.tri + 3u * (tBase + 8u * k + G.j);
+                const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+                g = __float_as_uint(a.w);
+                ok = tri_test(o, d, a, b, c, tmin, h.t, t, u, v) && (t < h.t || (t == h.t && g < h.gid));
+                // b.w != 0: the triangle's material has an alpha map
+                if (ok && __float_as_uint(b.w)) ok = alpha_pass(S, g, u, v, seed, key, false);
+            }
+            if (!__ballot_sync(G.mask, ok)) continue;
+            // the least (t, id) of the group (t + 0: one zero; its bits, mapped to order as t does)
+            const uint32_t bits = __float_as_uint(t + 0.0f), tb = bits ^ ((uint32_t)((int32_t)bits >> 31) | 0x80000000u);
+            const uint32_t tm = __reduce_min_sync(G.mask, ok ? tb : 0xFFFFFFFFu);
+            const uint32_t gm = __reduce_min_sync(G.mask, ok && tb == tm ? g : 0xFFFFFFFFu);
+            const uint32_t src = (uint32_t)__ffs(__ballot_sync(G.mask, ok && tb == tm && g == gm)) - 1u;
+            h.t = __shfl_sync(G.mask, t, src);
+            h.u = __shfl_sync(G.mask, u, src);
+            h.v = __shfl_sync(G.mask, v, src);
+            h.gid = gm;
+        }
+    } while (next_node8(S, K, r, gBase, gImask, gHits, sp, visits, child, err));
+    return h;
+}
+// Occlusion in scenes without glass.
+__device__ __forceinline__ bool trace_shadow8(const Group8 &G, const DevScene &S, float3 o, float3 d, float tmin,
+                                              float tmax, uint32_t *err, uint32_t seed, uint32_t key) {
+    if (S.numNodes == 0) return false;
+    TravStack K;
+    const RayPre r = ray_pre(o, d);
+    uint32_t gBase, gImask, gHits, tBase, tHits, visits = 1, child = 0;
+    int sp = 0;
+    do {
+        intersect_node8(G, S, child, r, tmin, tmax, gBase, gImask, gHits, tBase, tHits);
+        for (uint32_t k = 0; tHits >> (8u * k); k++) {
+            bool ok = (tHits >> (8u * k + G.j)) & 1u;
+            if (ok) {
+                const float4 *tp = S.tri + 3u * (tBase + 8u * k + G.j);
+                const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+                float t, u, v;
+                ok = tri_test(o, d, a, b, c, tmin, tmax, t, u, v);
+                if (ok && __float_as_uint(b.w)) ok = alpha_pass(S, __float_as_uint(a.w), u, v, seed, key, true);
+            }
+            if (__ballot_sync(G.mask, ok)) return true;
+        }
+    } while (next_node8(S, K, r, gBase, gImask, gHits, sp, visits, child, err));
+    return false;
 }
 
 }  // namespace pt

@@ -109,6 +109,8 @@ struct WaveArgs {
     unsigned long long *rayTotals;  // [0] extension, [1] shadow
     unsigned long long *tailRays;   // extension rays of k_tail (also in rayTotals[0])
     uint32_t *restLaunched;         // kernels launched by the conditional bodies after k_tail
+    uint32_t coopMax;               // queues of at most this many rays go to the 8-lanes-per-ray kernels
+    uint32_t coopTailMax;           // and tails of at most this many paths to k_tail8
     uint32_t tailMax;               // k_tail takes a wave's paths when at most this many are left
     uint32_t *err;
     uint32_t shadowCap;
@@ -358,7 +360,7 @@ template <bool CLASSIFY>
 __device__ __forceinline__ void finish_extend(const WaveArgs &A, uint32_t i, const Hit &h) {
     __stcs(A.qhit + i, make_float4(h.t, __uint_as_float(h.gid), h.u, h.v));
     if (CLASSIFY) {
-        int c = h.gid == 0xFFFFFFFFu ? (int)CLS_MISS : (int)__ldg(A.S.meshClass + __ldg(A.S.triMesh + h.gid));
+        int c = h.gid == 0xFFFFFFFFu ? (int)CLS_MISS : (int)__ldg(A.S.triClass + h.gid);
         class_append(A, c, i);
     }
 }
@@ -455,6 +457,7 @@ __device__ __forceinline__ void extend_queue(const WaveArgs &A) {
     // the queue (coherent traversal), and the class queues and the next ray
     // queue keep that order for the kernels that follow
     const uint32_t n = *(volatile uint32_t *)A.cntIn;
+    if (!MEDIA && n <= A.coopMax) return;  // k_extend8 takes it
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&A.rayTotals[0], (unsigned long long)n);
     PT_QUEUE_STACK(K)
     for (uint32_t base; (base = claim32(A.stealExt)) < n;) {
@@ -529,6 +532,7 @@ template <bool MEDIA_TR>
 __device__ __forceinline__ void shadow_queue(const WaveArgs &A) {
     // appends past the capacity were dropped (and flagged): only what was stored is read
     const uint32_t n = min(*(volatile uint32_t *)A.cntShadow, A.shadowCap);
+    if (!MEDIA_TR && n <= A.coopMax) return;  // k_shadow8 takes it
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&A.rayTotals[1], (unsigned long long)n);
     PT_QUEUE_STACK(K)
     for (uint32_t base; (base = claim32(A.stealShadow)) < n;) {
@@ -633,7 +637,7 @@ __global__ void __launch_bounds__(kBlock) k_classify(WaveArgs A) {
         const uint32_t gid = __float_as_uint(A.qhit[i].y);
         const int c = gid == 0xFFFFFFFFu ? (int)CLS_MISS
                       : (gid >> 31)      ? (int)CLS_MEDIUM
-                                         : (int)__ldg(A.S.meshClass + __ldg(A.S.triMesh + gid));
+                                         : (int)__ldg(A.S.triClass + gid);
         class_append(A, c, i);
     }
 }
@@ -699,6 +703,70 @@ __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_ratio(WaveArg
         if (s >> 31) __stcs(A.pendE + slot, out);
         else __stcs(A.pendA + slot, out);
         have = false;
+    }
+}
+// ---- short queues: 8 lanes per ray -------------------------------------------------
+// Launched beside k_extend / k_shadow; the queue's length decides on the
+// device which of the two does the work.  kCoopMax: the rays that are
+// resident at once with 8 lanes each (32 warps of 4 rays on 148 SMs).  64 x 64
+// room, 8 bounces: 0.41 -> 0.33 ms; 1280 x 720 preview, whose last bounces and
+// tail hold some 1,000 paths: 1.44 -> 1.22 ms.
+constexpr uint32_t kCoopMax = 148u * 32u * 4u;
+constexpr int kCoopBlock = 64;
+constexpr uint32_t kCoopTailMax = kCoopMax / 4;  // k_tail8: 8 blocks of 64 per SM (128 registers)
+__device__ __forceinline__ uint32_t claim4(uint32_t *next) {
+    uint32_t base = 0;
+    if (lane_id() == 0) base = atomicAdd(next, 4u);
+    return __shfl_sync(0xFFFFFFFFu, base, 0) + (lane_id() >> 3);
+}
+template <bool CLASSIFY>
+__global__ void __launch_bounds__(kCoopBlock) k_extend8(WaveArgs A) {
+    const uint32_t n = *(volatile uint32_t *)A.cntIn;
+    if (n > A.coopMax) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&A.rayTotals[0], (unsigned long long)n);
+    const Group8 G = group8();
+    for (uint32_t i = claim4(A.stealExt); __any_sync(0xFFFFFFFFu, i < n); i = claim4(A.stealExt)) {
+        if (i >= n) continue;
+        const float4 o = A.qoIn[i], d = A.qdIn[i];
+        uint32_t aseed = 0, akey = 0;
+        if (A.S.hasAlpha) {
+            const uint32_t slot = A.bounce == 0u ? i : A.qslotIn[i];
+            Rng r = load_rng(A, slot, A.rng[slot]);
+            aseed = alpha_seed(r.pixelSeed, r.sampleIndex);
+            akey = alpha_key(A.rng[slot].z, 0u);
+        }
+        const Hit h = trace_closest8(G, A.S, make_float3(o.x, o.y, o.z), make_float3(d.x, d.y, d.z), o.w, d.w, A.err,
+                                     aseed, akey);
+        if (G.j == 0) finish_extend<CLASSIFY>(A, i, h);
+        __syncwarp(G.mask);
+    }
+}
+__global__ void __launch_bounds__(kCoopBlock) k_shadow8(WaveArgs A) {
+    const uint32_t n = min(*(volatile uint32_t *)A.cntShadow, A.shadowCap);
+    if (n > A.coopMax) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&A.rayTotals[1], (unsigned long long)n);
+    const Group8 G = group8();
+    for (uint32_t i = claim4(A.stealShadow); __any_sync(0xFFFFFFFFu, i < n); i = claim4(A.stealShadow)) {
+        if (i >= n) continue;
+        const float4 o = A.so[i], d = A.sd[i];
+        const uint32_t s = A.sslot[i], slot = s & kShadowSlotMask;
+        uint32_t aseed = 0, akey = 0;
+        if (A.S.hasAlpha) {
+            Rng r = load_rng(A, slot, make_uint4(0u, 0u, 0u, 0u));  // seeds only
+            aseed = alpha_seed(r.pixelSeed, r.sampleIndex);
+            akey = alpha_key(A.rng[slot].z - 1u, (s >> 31) ? 2u : 1u);
+        }
+        const bool occ = trace_shadow8(G, A.S, make_float3(o.x, o.y, o.z), make_float3(d.x, d.y, d.z), o.w, d.w, A.err,
+                                       aseed, akey);
+        if (G.j == 0) {
+            const float4 X = A.sX[i], Th = A.sthr[i];
+            const float3 thr = make_float3(Th.x, Th.y, Th.z), tr = v3(1.0f);
+            const float3 R = occ ? thr * v3(0.0f) : thr * (make_float3(X.x, X.y, X.z) * tr);
+            const float4 out = make_float4(R.x, R.y, R.z, 0.0f);
+            if (s >> 31) A.pendE[slot] = out;
+            else A.pendA[slot] = out;
+        }
+        __syncwarp(G.mask);
     }
 }
 __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_shadow(WaveArgs A) { shadow_queue<false>(A); }
@@ -1008,19 +1076,17 @@ __device__ bool subsurface_walk(const WaveArgs &A, float3 pos, float3 dir, uint3
         float d = sigmaT > 0.0f ? -logf(mx(next_float(rng, S.sobol1), 1e-10f)) / sigmaT : 1e30f;
         Hit p = trace_closest(S, pos, dir, 1e-4f, d, A.err, aseed, alpha_key(bounce, 3u));
         if (p.gid != 0xFFFFFFFFu && p.t < d) {
-            const uint32_t hm = __ldg(S.triMesh + p.gid);
-            if (hm != mesh) {
+            const uint4 ti = __ldg(S.triIdx + p.gid);
+            const uint32_t i0 = ti.x, i1 = ti.y, i2 = ti.z;
+            if (ti.w != mesh) {
                 tmul = v3(0.0f);
                 return false;
             }
-            const uint32_t prim = p.gid - __ldg(S.meshFirstTri + hm);
-            uint32_t i0, i1, i2;
-            tri_vidx(S, hm, prim, i0, i1, i2);
             float3 bPos = pos + dir * p.t;
             float w0 = 1.0f - p.u - p.v;
-            float3 nn = ld3(S.nrm, i0) * w0 + ld3(S.nrm, i1) * p.u + ld3(S.nrm, i2) * p.v;
+            float3 nn = ld4(S.nrm4, i0) * w0 + ld4(S.nrm4, i1) * p.u + ld4(S.nrm4, i2) * p.v;
             float l2 = dot(nn, nn);
-            float3 p0 = ld3(S.pos, i0), p1 = ld3(S.pos, i1), p2 = ld3(S.pos, i2);
+            float3 p0 = ld4(S.pos4, i0), p1 = ld4(S.pos4, i1), p2 = ld4(S.pos4, i2);
             float3 Nb = normalize(l2 < 1e-8f ? normalize(cross(p1 - p0, p2 - p0)) : nn * (1.0f / sqrtf(l2)));
             if (dot(Nb, dir) < 0.0f) Nb = -Nb;
             float Fr = fresnel(dot(dir, Nb), intIOR, extIOR);
@@ -1061,10 +1127,9 @@ __device__ bool subsurface_walk(const WaveArgs &A, float3 pos, float3 dir, uint3
 // normal map in the frame of the triangle's UV derivatives, roughness (not
 // for hair, whose `roughness` is beta_m), specular (x 0.5), subsurface; each
 // at the mip level of the hit's UV footprint.  Overrides m's fields, bends N.
-__device__ __forceinline__ void apply_textures(const DevScene &S, pt_material &m, uint32_t mesh, uint32_t prim,
-                                               float hitT, uint32_t i0, uint32_t i1, uint32_t i2, float b1, float b2,
+__device__ __forceinline__ void apply_textures(const DevScene &S, pt_material &m, float hitT, uint32_t i0, uint32_t i1, uint32_t i2, float b1, float b2,
                                                float3 &N, uint32_t width, uint32_t height) {
-    const float foot = uv_footprint(S, mesh, prim, hitT, width, height);
+    const float foot = uv_footprint(S, i0, i1, i2, hitT, width, height);
     const float2 uv = interp_uv(S, i0, i1, i2, b1, b2);
     float3 alb = make_float3(m.albedo[0], m.albedo[1], m.albedo[2]);
     if (m.albedoTexIndex != PT_NO_TEXTURE) {
@@ -1072,7 +1137,7 @@ __device__ __forceinline__ void apply_textures(const DevScene &S, pt_material &m
         alb = make_float3(c.x, c.y, c.z);
     }
     if (m.normalTexIndex != PT_NO_TEXTURE) {
-        float3 p0 = ld3(S.pos, i0), p1 = ld3(S.pos, i1), p2 = ld3(S.pos, i2);
+        float3 p0 = ld4(S.pos4, i0), p1 = ld4(S.pos4, i1), p2 = ld4(S.pos4, i2);
         float3 e1 = p1 - p0, e2 = p2 - p0;
         float u0 = __ldg(S.uv + 2 * i0), v0 = __ldg(S.uv + 2 * i0 + 1);
         float du1 = __ldg(S.uv + 2 * i1) - u0, dv1 = __ldg(S.uv + 2 * i1 + 1) - v0;
@@ -1233,17 +1298,15 @@ __device__ __forceinline__ void shade_item(const WaveArgs &A, bool active, uint3
             if (lastPdf == 0.0f) Lo += thr * env;
             else Lo += thr * env * balance(lastPdf, env_pdf(S, A.envMode, rd));
         } else if (C != CLS_MISS) {
-            uint32_t mesh = __ldg(S.triMesh + gid);
-            uint32_t prim = gid - __ldg(S.meshFirstTri + mesh);
-            pt_material m = S.mats[mesh];
+            const uint4 ti = __ldg(S.triIdx + gid);
+            const uint32_t i0 = ti.x, i1 = ti.y, i2 = ti.z, mesh = ti.w;
+            pt_material m = load_material(S, mesh);
             const uint32_t type = C >= CLS_DIFFUSE ? class_type(C) : m.type;
-            uint32_t i0, i1, i2;
-            tri_vidx(S, mesh, prim, i0, i1, i2);
             float bx = h4.z, by = h4.w, w0 = 1.0f - bx - by;
             float3 hp = ro + rd * h4.x;
-            float3 p0 = ld3(S.pos, i0), p1 = ld3(S.pos, i1), p2 = ld3(S.pos, i2);
+            float3 p0 = ld4(S.pos4, i0), p1 = ld4(S.pos4, i1), p2 = ld4(S.pos4, i2);
             float3 Ng = normalize(normalize(cross(p1 - p0, p2 - p0)));
-            float3 nn = ld3(S.nrm, i0) * w0 + ld3(S.nrm, i1) * bx + ld3(S.nrm, i2) * by;
+            float3 nn = ld4(S.nrm4, i0) * w0 + ld4(S.nrm4, i1) * bx + ld4(S.nrm4, i2) * by;
             float l2 = dot(nn, nn);
             float3 N = normalize(l2 < 1e-8f ? normalize(cross(p1 - p0, p2 - p0)) : nn * (1.0f / sqrtf(l2)));
             bool back = dot(Ng, rd) > 0.0f;
@@ -1252,7 +1315,7 @@ __device__ __forceinline__ void shade_item(const WaveArgs &A, bool active, uint3
             if (TEX || (C == CLS_ANY && has_shading_textures(m)))
             {
                 const uint2 wh = path_image(A, slot);
-                apply_textures(S, m, mesh, prim, h4.x, i0, i1, i2, bx, by, N, wh.x, wh.y);
+                apply_textures(S, m, h4.x, i0, i1, i2, bx, by, N, wh.x, wh.y);
             }
             // Radiance cache: the first surface vertex after a rough bounce ends
             // the path (a query, resolved after the wave), or, with probability
@@ -1452,7 +1515,7 @@ __device__ __forceinline__ void shade_item(const WaveArgs &A, bool active, uint3
                             float3 aBlur = aSharp, detail = v3(1.0f);
                             if (m.albedoTexIndex != PT_NO_TEXTURE) {  // albedo blurred 4 mip levels up
                                 const uint2 wh = path_image(A, slot);
-                                const float foot = uv_footprint(S, mesh, prim, h4.x, wh.x, wh.y);
+                                const float foot = uv_footprint(S, i0, i1, i2, h4.x, wh.x, wh.y);
                                 const float2 tuv = interp_uv(S, i0, i1, i2, bx, by);
                                 float4 cb = tex_sample(S, m.albedoTexIndex, tuv.x, tuv.y,
                                                        tex_lod(S, m.albedoTexIndex, foot) + 4.0f);
@@ -1583,16 +1646,10 @@ __device__ __forceinline__ void tail_shadow(const WaveArgs &A, Stack &K, uint32_
     if (kind) __stcs(A.pendE + slot, out);
     else __stcs(A.pendA + slot, out);
 }
-// One shading event of queue position i with the per-bounce kernels' code.
-template <bool INLINE, class Stack>
-__device__ __forceinline__ void tail_shade(const WaveArgs &A, Stack &K, uint32_t i, ShadeOut &O, uint32_t &traced) {
-    if (INLINE) {
-        shade_item<true, CLS_ANY, false>(A, true, i, O);
-        traced += (O.neeA.traced ? 1u : 0u) + (O.neeE.traced ? 1u : 0u);
-        return;
-    }
-    const uint32_t gid = __float_as_uint(A.qhit[i].y);
-    const int c = gid == 0xFFFFFFFFu ? (int)CLS_MISS : (int)__ldg(A.S.meshClass + __ldg(A.S.triMesh + gid));
+// One shading event of queue position i (hit id gid) with the per-bounce
+// kernels' code.
+__device__ __forceinline__ void tail_event(const WaveArgs &A, uint32_t i, uint32_t gid, ShadeOut &O) {
+    const int c = gid == 0xFFFFFFFFu ? (int)CLS_MISS : (int)__ldg(A.S.triClass + gid);
     switch (c) {
         case CLS_MISS: shade_item<false, CLS_MISS, false>(A, true, i, O); break;
         case CLS_EMIT: shade_item<false, CLS_EMIT, false>(A, true, i, O); break;
@@ -1608,6 +1665,15 @@ __device__ __forceinline__ void tail_shade(const WaveArgs &A, Stack &K, uint32_t
         case CLS_TEX + CLS_DISNEY: shade_item<false, CLS_TEX + CLS_DISNEY, false>(A, true, i, O); break;
         default: shade_item<false, CLS_TEX + CLS_HAIR, false>(A, true, i, O); break;
     }
+}
+template <bool INLINE, class Stack>
+__device__ __forceinline__ void tail_shade(const WaveArgs &A, Stack &K, uint32_t i, ShadeOut &O, uint32_t &traced) {
+    if (INLINE) {
+        shade_item<true, CLS_ANY, false>(A, true, i, O);
+        traced += (O.neeA.traced ? 1u : 0u) + (O.neeE.traced ? 1u : 0u);
+        return;
+    }
+    tail_event(A, i, __float_as_uint(A.qhit[i].y), O);
     if (O.neeA.ray) {
         tail_shadow(A, K, O.slot, 0u, O.neeA, O.thrNee);
         ++traced;
@@ -1617,9 +1683,99 @@ __device__ __forceinline__ void tail_shade(const WaveArgs &A, Stack &K, uint32_t
         ++traced;
     }
 }
+// The tail of few paths: 8 lanes per path share its traversals; its first lane
+// alone runs the shading events and touches the path's state, the others get
+// their rays from it.
+__device__ __forceinline__ float3 from_first(const Group8 &G, float3 v) {
+    return make_float3(__shfl_sync(G.mask, v.x, G.shift), __shfl_sync(G.mask, v.y, G.shift),
+                       __shfl_sync(G.mask, v.z, G.shift));
+}
+// tail_shadow's work; `ne`, `thr` and `slot` are the first lane's.
+__device__ __forceinline__ void tail_shadow8(const WaveArgs &A, const Group8 &G, uint32_t slot, uint32_t kind,
+                                             const NeeOut &ne, float3 thr) {
+    uint32_t aseed = 0, akey = 0;
+    if (A.S.hasAlpha) {  // the shading event already advanced the path's bounce counter
+        if (G.j == 0) {
+            Rng r = load_rng(A, slot, A.rng[slot]);
+            aseed = alpha_seed(r.pixelSeed, r.sampleIndex);
+            akey = alpha_key(A.rng[slot].z - 1u, kind ? 2u : 1u);
+        }
+        aseed = __shfl_sync(G.mask, aseed, G.shift);
+        akey = __shfl_sync(G.mask, akey, G.shift);
+    }
+    const float3 o = from_first(G, ne.o), d = from_first(G, ne.d);
+    const float tmin = __shfl_sync(G.mask, ne.tmin, G.shift), tmax = __shfl_sync(G.mask, ne.tmax, G.shift);
+    const bool occ = trace_shadow8(G, A.S, o, d, tmin, tmax, A.err, aseed, akey);
+    if (G.j == 0) {
+        const float3 tr = v3(1.0f);
+        const float3 R = occ ? thr * v3(0.0f) : thr * (ne.X * tr);
+        const float4 out = make_float4(R.x, R.y, R.z, 0.0f);
+        if (kind) A.pendE[slot] = out;
+        else A.pendA[slot] = out;
+    }
+    __syncwarp(G.mask);
+}
+__global__ void __launch_bounds__(kCoopBlock, 8) k_tail8(const __grid_constant__ WaveArgs A) {
+    const uint32_t n = *(volatile uint32_t *)A.cntIn;
+    if (n > A.coopTailMax) return;
+    const Group8 G = group8();
+    uint32_t ext = 0, traced = 0;
+    for (uint32_t i = claim4(A.stealExt); __any_sync(0xFFFFFFFFu, i < n); i = claim4(A.stealExt)) {
+        bool live = i < n;
+        float4 o4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d4 = o4;
+        if (live) {
+            o4 = A.qoIn[i];
+            d4 = A.qdIn[i];
+        }
+        while (live) {
+            uint32_t aseed = 0, akey = 0;
+            if (A.S.hasAlpha) {
+                if (G.j == 0) {
+                    const uint32_t slot = A.bounce == 0u ? i : A.qslotIn[i];
+                    Rng r = load_rng(A, slot, A.rng[slot]);
+                    aseed = alpha_seed(r.pixelSeed, r.sampleIndex);
+                    akey = alpha_key(A.rng[slot].z, 0u);
+                }
+                aseed = __shfl_sync(G.mask, aseed, G.shift);
+                akey = __shfl_sync(G.mask, akey, G.shift);
+            }
+            const Hit h = trace_closest8(G, A.S, make_float3(o4.x, o4.y, o4.z), make_float3(d4.x, d4.y, d4.z), o4.w,
+                                         d4.w, A.err, aseed, akey);
+            ShadeOut O{};
+            uint32_t todo = 0;  // bit 0: the path goes on, 1 / 2: area / envmap NEE ray
+            if (G.j == 0) {
+                ++ext;
+                A.qhit[i] = make_float4(h.t, __uint_as_float(h.gid), h.u, h.v);
+                tail_event(A, i, h.gid, O);
+                todo = (O.cont ? 1u : 0u) | (O.neeA.ray ? 2u : 0u) | (O.neeE.ray ? 4u : 0u);
+                traced += __popc(todo >> 1);
+                o4 = make_float4(O.no.x, O.no.y, O.no.z, O.ntmin);
+                d4 = make_float4(O.nd.x, O.nd.y, O.nd.z, 1e20f);
+                if (O.cont) {
+                    A.qoIn[i] = o4;
+                    A.qdIn[i] = d4;
+                }
+            }
+            __syncwarp(G.mask);
+            todo = __shfl_sync(G.mask, todo, G.shift);
+            if (todo & 2u) tail_shadow8(A, G, O.slot, 0u, O.neeA, O.thrNee);
+            if (todo & 4u) tail_shadow8(A, G, O.slot, 1u, O.neeE, O.thrNee);
+            live = (todo & 1u) != 0u;
+            const float3 o = from_first(G, make_float3(o4.x, o4.y, o4.z)), d = from_first(G, make_float3(d4.x, d4.y, d4.z));
+            o4 = make_float4(o.x, o.y, o.z, __shfl_sync(G.mask, o4.w, G.shift));
+            d4 = make_float4(d.x, d.y, d.z, __shfl_sync(G.mask, d4.w, G.shift));
+        }
+        __syncwarp();
+    }
+    add_rays(A, 0, ext);  // (first lanes' counts)
+    add_rays(A, 1, traced);
+    for (int q = 16; q > 0; q >>= 1) ext += __shfl_xor_sync(0xFFFFFFFFu, ext, q);
+    if (lane_id() == 0 && ext) atomicAdd(A.tailRays, (unsigned long long)ext);
+}
 template <bool INLINE>
 __global__ void __launch_bounds__(kBlock, 2) k_tail(const __grid_constant__ WaveArgs A) {
     const uint32_t n = *(volatile uint32_t *)A.cntIn;
+    if (!INLINE && n <= A.coopTailMax) return;  // k_tail8 has them
     if (n > A.tailMax) return;  // uniform: the per-bounce kernels take the rest
     PT_QUEUE_STACK(K)
     uint32_t ext = 0, traced = 0;
@@ -1959,7 +2115,11 @@ bool enqueue_rest_conditional(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32
 // Which walks through media run in their own kernels: free flights where a
 // medium is heterogeneous, the ratio tracking of deferred NEE rays except in
 // scenes with glass (whose shadow rays carry a transmission of their own).
+// And which rays go to the 8-lanes-per-ray kernels (none with glass, whose
+// shadow rays multiply transmissions in traversal order).
 void media_passes(const pt_ctx *ctx, WaveArgs &A) {
+    A.coopMax = A.S.hasGlass ? 0u : kCoopMax;
+    A.coopTailMax = A.S.hasGlass || ctx->dbgTail == 1u ? 0u : kCoopTailMax;
     A.flightPass = ctx->hasHetero ? 1u : 0u;
     A.ratioPass = A.S.mediaTrDeferred && !A.S.hasGlass ? 1u : 0u;
 }
@@ -1995,6 +2155,27 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         if (shadowOpen) chk(cudaStreamWaitEvent(st, fj->joinEv[0], 0));
         shadowOpen = false;
     };
+    // The two forms of a traversal kernel over a queue of at most `most` rays
+    // (`exact`: of just that many), `one` a lane per ray and `eight` 8 lanes:
+    // the queue's length decides on the device, so both are launched where it
+    // is not known here; in a capture `eight` on branch br, beside `one`.
+    const unsigned coopGrid = (unsigned)std::min<uint64_t>(2ull * A.waveCount, kCoopMax) * 8u / kCoopBlock + 1u;
+    auto both = [&](uint64_t most, bool exact, cudaStream_t s, int br, auto one, auto eight) {
+        const bool useOne = most > A.coopMax, useEight = A.coopMax && !(exact && useOne);
+        const bool apart = fj && useOne && useEight;
+        cudaStream_t s8 = s;
+        if (apart) {
+            s8 = fj->branch[br];
+            chk(cudaEventRecord(fj->forkEv, s));
+            chk(cudaStreamWaitEvent(s8, fj->forkEv, 0));
+        }
+        if (useOne) one(s);
+        if (useEight) eight(s8);
+        if (apart) {
+            chk(cudaEventRecord(fj->joinEv[br], s8));
+            chk(cudaStreamWaitEvent(s, fj->joinEv[br], 0));
+        }
+    };
     for (uint32_t b = first; b < depth; b++) {
         const int cur = (int)(b & 1u);
         uint32_t *cnt = B.counters + (size_t)(1 + b) * kCounterWords;
@@ -2015,7 +2196,10 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
             WaveArgs T = A;  // a path's flights run in its own thread
             T.flightPass = 0u;
             if (inl) k_tail<true><<<G.tailI, kBlock, 0, st>>>(T);
-            else k_tail<false><<<G.tail, kBlock, 0, st>>>(A);
+            else {
+                k_tail<false><<<G.tail, kBlock, 0, st>>>(A);
+                if (A.coopTailMax) k_tail8<<<kCoopTailMax * 8u / kCoopBlock, kCoopBlock, 0, st>>>(A);
+            }
             if (fj) {
                 if (enqueue_rest_conditional(ctx, E, A, b, depth, G, err)) return err;
             }
@@ -2031,7 +2215,8 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         if (inl) {
             const Shape x = shape(G.ext, A.waveCount), h = shape(G.shadeI, A.waveCount);
             E.begin(STG_EXTEND);
-            k_extend<false><<<x.grid, x.block, 0, st>>>(A);
+            both(A.waveCount, b == 0, st, 1, [&](cudaStream_t s) { k_extend<false><<<x.grid, x.block, 0, s>>>(A); },
+                 [&](cudaStream_t s) { k_extend8<false><<<coopGrid, kCoopBlock, 0, s>>>(A); });
             E.end();
             if (A.flightPass) {
                 const Shape f = shape(G.flight, A.waveCount);
@@ -2047,7 +2232,8 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         E.begin(STG_EXTEND);
         if (A.flightPass) {
             const Shape x = shape(G.ext, A.waveCount), f = shape(G.flight, A.waveCount);
-            k_extend<false><<<x.grid, x.block, 0, st>>>(A);
+            both(A.waveCount, b == 0, st, 1, [&](cudaStream_t s) { k_extend<false><<<x.grid, x.block, 0, s>>>(A); },
+                 [&](cudaStream_t s) { k_extend8<false><<<coopGrid, kCoopBlock, 0, s>>>(A); });
             E.end();
             E.begin(STG_EXTEND);
             k_flight<<<f.grid, f.block, 0, st>>>(A);
@@ -2059,7 +2245,8 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
             k_extend_media<<<x.grid, x.block, 0, st>>>(A);
         } else {
             const Shape x = shape(G.extC, A.waveCount);
-            k_extend<true><<<x.grid, x.block, 0, st>>>(A);
+            both(A.waveCount, b == 0, st, 1, [&](cudaStream_t s) { k_extend<true><<<x.grid, x.block, 0, s>>>(A); },
+                 [&](cudaStream_t s) { k_extend8<true><<<coopGrid, kCoopBlock, 0, s>>>(A); });
         }
         E.end();
         joinShadow();  // the shading pass folds its results in
@@ -2097,7 +2284,9 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         const Shape w = shape(A.S.mediaTrDeferred ? G.shadowM : G.shadow, 2ull * A.waveCount);
         E.begin(STG_SHADOW);
         if (A.S.mediaTrDeferred) k_shadow_media<<<w.grid, w.block, 0, ss>>>(A);
-        else k_shadow<<<w.grid, w.block, 0, ss>>>(A);
+        else
+            both(2ull * A.waveCount, false, ss, 2, [&](cudaStream_t s) { k_shadow<<<w.grid, w.block, 0, s>>>(A); },
+                 [&](cudaStream_t s) { k_shadow8<<<coopGrid, kCoopBlock, 0, s>>>(A); });
         E.end();
         if (A.ratioPass) {
             const Shape q = shape(G.ratio, 2ull * A.waveCount);
