@@ -526,6 +526,7 @@ int pt_destroy(pt_ctx *ctx) {
     pt_branch_free(ctx);
     ctx->free_scene();
     ctx->sceneMem.release();
+    ctx->buildMem.release();
     pt_wave_free(ctx);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->d_sobol1) cudaFree(ctx->d_sobol1);
@@ -859,16 +860,14 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         PT_CUDA(ctx->alloc_scene(&dcguide, (size_t)H * (kCdfGuide + 1)));
     }
     {
-        // temporaries, one allocation: RGB texels, sin table, row sums, FP64 weights, Vose scratch
+        // temporaries (build workspace): RGB texels, sin table, row sums, FP64 weights, Vose scratch
         const bool blocks = W <= kEnvRowMax && H <= kEnvRowMax;
         const size_t most = std::max<size_t>(WH, H);
-        DeviceArena tmp;
+        DeviceArena &tmp = ctx->buildMem;
         float *drgb = nullptr;
         double *wall, *rowSum, *q = nullptr, *total;
         uint32_t *stk = nullptr;
-        void *first;
-        cudaError_t e = tmp.alloc(&first, WH * (12 + 8) + (blocks ? 0 : most * 12) + (size_t)H * 16 + 16 + 8 * 256);
-        if (e == cudaSuccess) tmp.chunks[0].used = 0;
+        cudaError_t e = tmp.begin(WH * (12 + 8) + (blocks ? 0 : most * 12) + (size_t)H * 16 + 16 + 8 * 256);
         auto ta = [&](auto **p, size_t bytes) { if (e == cudaSuccess) e = tmp.alloc((void **)p, bytes); };
         ta(&drgb, WH * 12);
         ta(&wall, WH * 8);
@@ -880,11 +879,11 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
             ta(&q, most * 8);
             ta(&stk, most * 4);
         }
-        if (e != cudaSuccess) { tmp.release(); return ctx->fail(PT_E_NOMEM, "envmap temporaries"); }
+        if (e != cudaSuccess) return ctx->fail(PT_E_NOMEM, "envmap temporaries");
         const float black[3] = {0.0f, 0.0f, 0.0f};
         rc = h2d(drgb, haveEnv ? d->env_rgb : black, WH * 12);
         if (!rc) rc = h2d(dsin, sinRow.data(), (size_t)H * 4);
-        if (rc) { tmp.release(); return rc; }
+        if (rc) return rc;
         k_env_expand<<<(unsigned)std::min<size_t>((WH + 255) / 256, 4096), 256, 0, st>>>(WH, drgb, denv);
         if (blocks) {
             const size_t mostW = (size_t)W * 12, mostH = (size_t)H * 12;
@@ -904,7 +903,7 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         if (dmguide) k_env_guides<<<256, 256, 0, st>>>(W, H, dmarg, dcond, dmguide, dcguide);
         e = cudaGetLastError();
         const cudaError_t es = cudaStreamSynchronize(st);
-        tmp.release();
+        tmp.rewind();
         if (e == cudaSuccess) e = es;
         if (e != cudaSuccess) return ctx->fail(PT_E_CUDA, "envmap tables", cudaGetErrorString(e));
     }

@@ -811,15 +811,16 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
     PT_CUDA(ctx->alloc_scene(&codesS, n));
     PT_CUDA(ctx->alloc_scene(&idsS, n));
     PT_CUDA(ctx->alloc_scene(&children, 2 * (size_t)max(n - 1, 1u)));
-    // temporaries: one allocation, about 230 bytes per triangle and the sort's
-    // tile counts, given back before the build returns
-    DeviceArena tmp;
-    auto cleanup = [&]() { tmp.release(); };
+    // temporaries, in the context's build workspace
+    DeviceArena &tmp = ctx->buildMem;
+    auto cleanup = [&]() { tmp.rewind(); };
+    // (planFirst: which collapse is tried first, below)
+    int l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
+    const bool planFirst = ctx->dbgWidePlan || (uint64_t)n * 71u > (uint64_t)(l2 > 0 ? l2 : 126 << 20);
     {
-        void *all;
-        cudaError_t e = tmp.alloc(&all, (size_t)n * 232 + ((size_t)n / kRsTile + 1) * 1024 + 16384);
+        const cudaError_t e = tmp.begin((size_t)n * (planFirst ? 230 : 188) + ((size_t)n / kRsTile + 1) * 1024 + 16384);
         if (e != cudaSuccess) return ctx->fail(PT_E_NOMEM, "bvh temp", cudaGetErrorString(e));
-        tmp.chunks[0].used = 0;
     }
 #define TA(p, bytes)                                                                   \
     do {                                                                               \
@@ -874,9 +875,8 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
     const size_t ni = (size_t)max(n - 1, 1u);
     TA(cnt, ni * 4); TA(cost, ni * 4); TA(rewired, 4);
     TA(tch, ni * 8); TA(tip, ni * 4); TA(tlp, (size_t)n * 4);
-    float *planCost;
-    uint8_t *planSlots, *planWide;
-    TA(planCost, ni * 8 * 4); TA(planSlots, ni * 8); TA(planWide, ni);
+    float *planCost = nullptr;  // allocated when a plan is made
+    uint8_t *planSlots = nullptr, *planWide = nullptr;
     if (n > 1) {
         k_range_count<<<(n - 1 + B - 1) / B, B, 0, st>>>((int)n, rf, rl, cnt);
         cudaMemcpyAsync(tch, children, (size_t)(n - 1) * 8, cudaMemcpyDeviceToDevice, st);
@@ -915,9 +915,6 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
     // traversal stack is collapsed the other way, and only then does the
     // build fall back to the radix tree (its depth is bounded by the key
     // bits plus the index bits of equal keys).
-    int l2 = 0;
-    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
-    const bool planFirst = ctx->dbgWidePlan || (uint64_t)n * 71u > (uint64_t)(l2 > 0 ? l2 : 126 << 20);
     uint32_t cnt4[4];
     for (int attempt = 0; attempt < 3; attempt++) {
         const bool radix = attempt == 2 || n == 1;
@@ -930,6 +927,9 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
         }
         const uint8_t *plan = nullptr, *planW = nullptr;
         if (usePlan && n > 1) {  // the collapse plan of the restructured tree
+            TA(planCost, ni * 8 * 4);
+            TA(planSlots, ni * 8);
+            TA(planWide, ni);
             cudaMemsetAsync(flags, 0, (size_t)(n - 1) * 4, st);
             k_wide_plan<<<G, B, 0, st>>>((int)n, radix ? children : tch, radix ? intParent : tip,
                                          radix ? leafParent : tlp, cnt, intLo, intHi, planCost, planSlots,

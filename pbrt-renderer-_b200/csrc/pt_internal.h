@@ -193,6 +193,20 @@ struct DeviceArena {
         if (e == cudaSuccess) chunks.push_back(c);
         return e;
     }
+    // One chunk of at least `bytes`, empty (a workspace's start).
+    cudaError_t begin(size_t bytes) {
+        if (chunks.size() != 1 || chunks[0].size < bytes) {
+            release();
+            void *p;
+            const cudaError_t e = alloc(&p, bytes);
+            if (e != cudaSuccess) return e;
+        }
+        rewind();
+        return cudaSuccess;
+    }
+    void rewind() {
+        for (Chunk &c : chunks) c.used = 0;
+    }
     void reset() {
         size_t size = 0, used = 0;
         for (Chunk &c : chunks) { size += c.size; used += c.used; c.used = 0; }
@@ -235,6 +249,10 @@ struct pt_ctx {
     bool branchesReady = false;
     std::string err;
     DeviceArena sceneMem{(size_t)1 << 20};  // the uploaded scene's arrays
+    // workspace of uploads (about 190 bytes a triangle), kept for the next one
+    // until the wave buffers have to grow: mapping and unmapping it took from 1
+    // to 200 ms per upload, whatever else the driver was doing
+    DeviceArena buildMem;
     pt::DevScene S{};
     bool hasScene = false;
     uint32_t clsMask = 0;  // bit c: shading class c occurs in the scene

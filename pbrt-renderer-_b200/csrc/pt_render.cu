@@ -1905,6 +1905,7 @@ static_assert(kWaveBytesPerPath == 364, "wave state layout");
 
 static int wave_alloc(pt_ctx *ctx, size_t cap) {
     if (ctx->W.cap >= cap) return PT_OK;
+    ctx->buildMem.release();
     pt_wave_free(ctx);
     WaveBuffers &W = ctx->W;
     size_t sc = 2 * cap;
@@ -2155,26 +2156,21 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         if (shadowOpen) chk(cudaStreamWaitEvent(st, fj->joinEv[0], 0));
         shadowOpen = false;
     };
-    // The two forms of a traversal kernel over a queue of at most `most` rays
-    // (`exact`: of just that many), `one` a lane per ray and `eight` 8 lanes:
-    // the queue's length decides on the device, so both are launched where it
-    // is not known here; in a capture `eight` on branch br, beside `one`.
+    // The two forms of a traversal kernel over a queue of at most `most` rays,
+    // `one` a lane per ray and `eight` 8 lanes: the queue's length decides on
+    // the device, so both are launched where it is not known here.  `eight` is
+    // left out where the queue is hardly that short yet (a quarter of the paths
+    // going on at each bounce), and `one` then takes queues of any length.
+    // (As parallel nodes they saved no time, and the wider graph took 3 ms more
+    // to instantiate.)
     const unsigned coopGrid = (unsigned)std::min<uint64_t>(2ull * A.waveCount, kCoopMax) * 8u / kCoopBlock + 1u;
-    auto both = [&](uint64_t most, bool exact, cudaStream_t s, int br, auto one, auto eight) {
-        const bool useOne = most > A.coopMax, useEight = A.coopMax && !(exact && useOne);
-        const bool apart = fj && useOne && useEight;
-        cudaStream_t s8 = s;
-        if (apart) {
-            s8 = fj->branch[br];
-            chk(cudaEventRecord(fj->forkEv, s));
-            chk(cudaStreamWaitEvent(s8, fj->forkEv, 0));
-        }
-        if (useOne) one(s);
-        if (useEight) eight(s8);
-        if (apart) {
-            chk(cudaEventRecord(fj->joinEv[br], s8));
-            chk(cudaStreamWaitEvent(s, fj->joinEv[br], 0));
-        }
+    const uint32_t coopMax = A.coopMax;
+    auto both = [&](uint64_t most, auto one, auto eight) {
+        const bool useEight = coopMax && (A.bounce > 15u || (A.waveCount >> (2u * A.bounce)) <= coopMax);
+        A.coopMax = useEight ? coopMax : 0u;
+        if (most > A.coopMax) one();
+        if (useEight) eight();
+        A.coopMax = coopMax;
     };
     for (uint32_t b = first; b < depth; b++) {
         const int cur = (int)(b & 1u);
@@ -2215,8 +2211,8 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         if (inl) {
             const Shape x = shape(G.ext, A.waveCount), h = shape(G.shadeI, A.waveCount);
             E.begin(STG_EXTEND);
-            both(A.waveCount, b == 0, st, 1, [&](cudaStream_t s) { k_extend<false><<<x.grid, x.block, 0, s>>>(A); },
-                 [&](cudaStream_t s) { k_extend8<false><<<coopGrid, kCoopBlock, 0, s>>>(A); });
+            both(A.waveCount, [&] { k_extend<false><<<x.grid, x.block, 0, st>>>(A); },
+                 [&] { k_extend8<false><<<coopGrid, kCoopBlock, 0, st>>>(A); });
             E.end();
             if (A.flightPass) {
                 const Shape f = shape(G.flight, A.waveCount);
@@ -2232,8 +2228,8 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         E.begin(STG_EXTEND);
         if (A.flightPass) {
             const Shape x = shape(G.ext, A.waveCount), f = shape(G.flight, A.waveCount);
-            both(A.waveCount, b == 0, st, 1, [&](cudaStream_t s) { k_extend<false><<<x.grid, x.block, 0, s>>>(A); },
-                 [&](cudaStream_t s) { k_extend8<false><<<coopGrid, kCoopBlock, 0, s>>>(A); });
+            both(A.waveCount, [&] { k_extend<false><<<x.grid, x.block, 0, st>>>(A); },
+                 [&] { k_extend8<false><<<coopGrid, kCoopBlock, 0, st>>>(A); });
             E.end();
             E.begin(STG_EXTEND);
             k_flight<<<f.grid, f.block, 0, st>>>(A);
@@ -2245,8 +2241,8 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
             k_extend_media<<<x.grid, x.block, 0, st>>>(A);
         } else {
             const Shape x = shape(G.extC, A.waveCount);
-            both(A.waveCount, b == 0, st, 1, [&](cudaStream_t s) { k_extend<true><<<x.grid, x.block, 0, s>>>(A); },
-                 [&](cudaStream_t s) { k_extend8<true><<<coopGrid, kCoopBlock, 0, s>>>(A); });
+            both(A.waveCount, [&] { k_extend<true><<<x.grid, x.block, 0, st>>>(A); },
+                 [&] { k_extend8<true><<<coopGrid, kCoopBlock, 0, st>>>(A); });
         }
         E.end();
         joinShadow();  // the shading pass folds its results in
@@ -2285,8 +2281,8 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         E.begin(STG_SHADOW);
         if (A.S.mediaTrDeferred) k_shadow_media<<<w.grid, w.block, 0, ss>>>(A);
         else
-            both(2ull * A.waveCount, false, ss, 2, [&](cudaStream_t s) { k_shadow<<<w.grid, w.block, 0, s>>>(A); },
-                 [&](cudaStream_t s) { k_shadow8<<<coopGrid, kCoopBlock, 0, s>>>(A); });
+            both(2ull * A.waveCount, [&] { k_shadow<<<w.grid, w.block, 0, ss>>>(A); },
+                 [&] { k_shadow8<<<coopGrid, kCoopBlock, 0, ss>>>(A); });
         E.end();
         if (A.ratioPass) {
             const Shape q = shape(G.ratio, 2ull * A.waveCount);
@@ -2423,6 +2419,7 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
             cap = want;
         } else {
             size_t freeB = 0, totalB = 0;
+            ctx->buildMem.release();
             if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) freeB = (size_t)4 << 30;
             size_t fit = (freeB / 2 + ctx->W.cap * kWaveBytesPerPath / 2) / kWaveBytesPerPath;
             cap = std::max<size_t>(std::min(want, fit), std::min<size_t>(want, (size_t)1 << 16));
@@ -2723,6 +2720,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
     cap = (size_t)std::min<uint64_t>(cap, total);
     if (cap > ctx->W.cap) {  // grow within half the free memory, as a single render does
         size_t freeB = 0, totalB = 0;
+        ctx->buildMem.release();
         if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) freeB = (size_t)4 << 30;
         size_t fit = (freeB / 2 + ctx->W.cap * kWaveBytesPerPath / 2) / (kWaveBytesPerPath + 8);
         cap = std::max<size_t>(std::min(cap, fit), std::min<size_t>(cap, (size_t)1 << 16));
