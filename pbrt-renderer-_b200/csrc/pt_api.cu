@@ -523,7 +523,8 @@ int pt_destroy(pt_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     pt_graph_free(ctx);
     pt_batch_free(ctx);
-    pt_branch_free(ctx);
+    pt_branch_free(ctx, 0);
+    pt_branch_free(ctx, 1);
     ctx->free_scene();
     ctx->sceneMem.release();
     ctx->buildMem.release();

@@ -243,10 +243,12 @@ struct pt_ctx {
     // branches of a captured render (ForkJoin in pt_render.cu): streams and
     // events that take part in captures only; [1]: of a conditional node's
     // body, which is a capture of its own on bodyStream
-    static constexpr int kBranches = 6;
+    // (one branch: with three a 64 x 64 room's call took 0.34 ms instead of 0.35,
+    // but the wider graph of a new context's first call 1 ms more)
+    static constexpr int kBranches = 1;
     cudaStream_t branch[2][kBranches] = {}, bodyStream = nullptr;
     cudaEvent_t forkEv[2] = {}, joinEv[2][kBranches] = {};
-    bool branchesReady = false;
+    bool branchesReady[2] = {false, false};
     std::string err;
     DeviceArena sceneMem{(size_t)1 << 20};  // the uploaded scene's arrays
     // workspace of uploads (about 190 bytes a triangle), kept for the next one
@@ -372,5 +374,5 @@ cudaError_t rc_enqueue_targets(pt_ctx *ctx, cudaStream_t st, float4 *lo_eta, uin
 cudaError_t rc_enqueue_train(pt_ctx *ctx, cudaStream_t st, uint32_t s, bool adam);
 constexpr uint32_t kRcStepsPerCall = 4;  // Adam steps per cached render call, on interleaved quarters of its records
 void pt_graph_free(pt_ctx *ctx);
-void pt_branch_free(pt_ctx *ctx);
+void pt_branch_free(pt_ctx *ctx, int k);
 void pt_batch_free(pt_ctx *ctx);

@@ -1997,21 +1997,20 @@ struct ForkJoin {
     cudaEvent_t forkEv;
     const cudaEvent_t *joinEv;
 };
-bool branches_ready(pt_ctx *ctx) {
-    if (ctx->branchesReady) return true;
-    bool ok = cudaStreamCreateWithFlags(&ctx->bodyStream, cudaStreamNonBlocking) == cudaSuccess;
-    for (int k = 0; k < 2; k++) {
-        ok = ok && cudaEventCreateWithFlags(&ctx->forkEv[k], cudaEventDisableTiming) == cudaSuccess;
-        for (int i = 0; i < pt_ctx::kBranches; i++) {
-            ok = ok && cudaStreamCreateWithFlags(&ctx->branch[k][i], cudaStreamNonBlocking) == cudaSuccess;
-            ok = ok && cudaEventCreateWithFlags(&ctx->joinEv[k][i], cudaEventDisableTiming) == cudaSuccess;
-        }
+// Set k (0: the render's, 1: a conditional body's) is made when first needed.
+bool branches_ready(pt_ctx *ctx, int k) {
+    if (ctx->branchesReady[k]) return true;
+    bool ok = cudaEventCreateWithFlags(&ctx->forkEv[k], cudaEventDisableTiming) == cudaSuccess;
+    if (k == 1) ok = ok && cudaStreamCreateWithFlags(&ctx->bodyStream, cudaStreamNonBlocking) == cudaSuccess;
+    for (int i = 0; i < pt_ctx::kBranches; i++) {
+        ok = ok && cudaStreamCreateWithFlags(&ctx->branch[k][i], cudaStreamNonBlocking) == cudaSuccess;
+        ok = ok && cudaEventCreateWithFlags(&ctx->joinEv[k][i], cudaEventDisableTiming) == cudaSuccess;
     }
     if (!ok) {
         cudaGetLastError();
-        pt_branch_free(ctx);
+        pt_branch_free(ctx, k);
     }
-    ctx->branchesReady = ok;
+    ctx->branchesReady[k] = ok;
     return ok;
 }
 
@@ -2073,6 +2072,7 @@ bool enqueue_rest_conditional(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32
                               const Grids &G, cudaError_t &err) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
+    if (!branches_ready(const_cast<pt_ctx *>(ctx), 1)) return false;
     if (cudaStreamGetCaptureInfo_v2(E.st, &cs, nullptr, &graph) != cudaSuccess || cs != cudaStreamCaptureStatusActive)
         return false;
     cudaGraphConditionalHandle h = 0;
@@ -2381,20 +2381,18 @@ bool graph_matches(const pt_ctx *ctx, const pt_render_params *P, size_t cap, con
 }
 }  // namespace
 
-void pt_branch_free(pt_ctx *ctx) {
-    for (int k = 0; k < 2; k++) {
-        for (int i = 0; i < pt_ctx::kBranches; i++) {
-            if (ctx->branch[k][i]) cudaStreamDestroy(ctx->branch[k][i]);
-            if (ctx->joinEv[k][i]) cudaEventDestroy(ctx->joinEv[k][i]);
-            ctx->branch[k][i] = nullptr;
-            ctx->joinEv[k][i] = nullptr;
-        }
-        if (ctx->forkEv[k]) cudaEventDestroy(ctx->forkEv[k]);
-        ctx->forkEv[k] = nullptr;
+void pt_branch_free(pt_ctx *ctx, int k) {
+    for (int i = 0; i < pt_ctx::kBranches; i++) {
+        if (ctx->branch[k][i]) cudaStreamDestroy(ctx->branch[k][i]);
+        if (ctx->joinEv[k][i]) cudaEventDestroy(ctx->joinEv[k][i]);
+        ctx->branch[k][i] = nullptr;
+        ctx->joinEv[k][i] = nullptr;
     }
-    if (ctx->bodyStream) cudaStreamDestroy(ctx->bodyStream);
-    ctx->bodyStream = nullptr;
-    ctx->branchesReady = false;
+    if (ctx->forkEv[k]) cudaEventDestroy(ctx->forkEv[k]);
+    ctx->forkEv[k] = nullptr;
+    if (k == 1 && ctx->bodyStream) cudaStreamDestroy(ctx->bodyStream);
+    if (k == 1) ctx->bodyStream = nullptr;
+    ctx->branchesReady[k] = false;
 }
 
 void pt_graph_free(pt_ctx *ctx) {
@@ -2504,7 +2502,7 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     bool useGraph = !timing;
     if (useGraph && !graph_matches(ctx, P, cap, d_sum, d_comp, A)) {
         pt_graph_free(ctx);
-        const bool forkOk = branches_ready(ctx);
+        const bool forkOk = branches_ready(ctx, 0);
         Enqueue E{ctx->ownStream, false, {}, 0};
         const ForkJoin fj{ctx->branch[0], ctx->forkEv[0], ctx->joinEv[0]};
         if (forkOk) E.fj = &fj;
@@ -2850,7 +2848,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
     if (!Bt.exec || Bt.key != key) {
         if (Bt.exec) cudaGraphExecDestroy(Bt.exec);
         Bt.exec = nullptr;
-        const bool forkOk = branches_ready(ctx);
+        const bool forkOk = branches_ready(ctx, 0);
         Enqueue E{ctx->ownStream, false, {}, 0};
         const ForkJoin fj{ctx->branch[0], ctx->forkEv[0], ctx->joinEv[0]};
         if (forkOk) E.fj = &fj;
