@@ -245,6 +245,7 @@ __global__ void k_refit(int n, const uint32_t *__restrict__ sorted, const float4
     for (int guard = 0; node >= 0 && guard < n; guard++) {
         __threadfence();
         if (atomicAdd(&flags[node], 1u) == 0u) return;  // first arrival: sibling finishes the node
+        __threadfence();  // both subtrees' bounds, after both arrivals
         int c0 = children[2 * node], c1 = children[2 * node + 1];
         float4 l0 = c0 >= 0 ? __ldcg(&intLo[c0]) : __ldcg(&leafLo[~c0]);
         float4 h0 = c0 >= 0 ? __ldcg(&intHi[c0]) : __ldcg(&leafHi[~c0]);
@@ -514,6 +515,9 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelet(TreeletIn T) {
                 tris = n0 + n1;
             }
         }
+        // What the owners' fences let them see of the subtrees, the whole warp
+        // sees after this barrier (votes and shuffles order no memory).
+        __syncwarp();
         for (uint32_t todo = __ballot_sync(kAll, node >= 0 && tris >= kTreeletMinTris); todo; todo &= todo - 1u) {
             const int src = __ffs(todo) - 1;
             const float r = treelet_restructure(T, W, __shfl_sync(kAll, node, src), __shfl_sync(kAll, c0, src),
@@ -525,9 +529,10 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelet(TreeletIn T) {
             T.cnt[node] = tris;
             node = __ldcg(&T.intParent[node]);
         }
-        // every lane's writes, before the owner of a node counts itself in at its parent
-        __threadfence();
+        // every lane's writes, before the owner of a node counts itself in at
+        // its parent: its fence has to come after the barrier to cover them
         __syncwarp();
+        __threadfence();
     }
 }
 
@@ -552,6 +557,7 @@ __global__ void k_wide_plan(int n, const int32_t *__restrict__ children, const i
     for (int guard = 0; node >= 0 && guard < n; guard++) {
         __threadfence();
         if (atomicAdd(&flags[node], 1u) == 0u) return;  // first arrival: sibling finishes the node
+        __threadfence();  // both subtrees' costs, after both arrivals
         float *cn = cost + 8 * (size_t)node;
         uint8_t *pn = plan + 8 * (size_t)node;
         if (cnt[node] <= kLeafMax) {
