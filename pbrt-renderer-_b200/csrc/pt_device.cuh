@@ -787,8 +787,11 @@ __device__ __forceinline__ void intersect_node(const DevScene &S, uint32_t ni, c
         unpack2(fma2(planes(i < 4 ? lza : lzb, i < 4 ? hza : hzb, sel, false), Sz, Oz), tnz, tfz);
         const float t0 = fmax3(tnx, tny, fmaxf(tnz, tmin));
         const float t1 = fmin3(tfx, tfy, fminf(tfz, tmax));
-        // missed where t0 > t1 x (1 + 2^-22): the difference's sign bit
-        miss = __funnelshift_l(__float_as_uint(__fadd_rn(__fmul_rn(t1, 1.00000024f), -t0)), miss, 1);
+        // missed where t0 > t1 x (1 + 2^-22): the difference's sign bit.  The
+        // product is rounded by an FMA with +0, which leaves no -0: a box that
+        // ends at t = -0 (a ray that leaves its lower plane) where the ray
+        // begins at +0 would otherwise differ by -0 and count as missed.
+        miss = __funnelshift_l(__float_as_uint(__fadd_rn(__fmaf_rn(t1, 1.00000024f, 0.0f), -t0)), miss, 1);
     }
     const uint32_t hit = ~miss & 0xFFu;
     // internal children: bit i to bit i ^ oct by three conditional swaps
