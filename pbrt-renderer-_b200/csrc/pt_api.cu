@@ -888,9 +888,19 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         k_env_expand<<<(unsigned)std::min<size_t>((WH + 255) / 256, 4096), 256, 0, st>>>(WH, drgb, denv);
         if (blocks) {
             const size_t mostW = (size_t)W * 12, mostH = (size_t)H * 12;
-            if (mostW > 48 * 1024) cudaFuncSetAttribute(k_alias_row_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mostW);
-            if ((size_t)W * 8 > 48 * 1024) cudaFuncSetAttribute(k_env_row_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W * 8));
-            if (mostH > 48 * 1024) cudaFuncSetAttribute(k_env_marginal_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mostH);
+            // The limit belongs to the kernel on this device, not to this context:
+            // always the most any map needs, so that an upload on another thread
+            // never lowers it between this and the launches.  (Without it the
+            // limit is 48 KB with the kernels' static variables counted in.)
+            auto limit = [&](auto *kernel, uint32_t bytesPerTexel) {
+                if (e == cudaSuccess)
+                    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(bytesPerTexel * kEnvRowMax));
+            };
+            limit(k_env_row_block, 8);
+            limit(k_env_marginal_block, 12);
+            limit(k_alias_row_block, 12);
+            if (e != cudaSuccess) return ctx->fail(PT_E_CUDA, "envmap kernel attributes", cudaGetErrorString(e));
             k_env_row_block<<<H, kEnvThreads, (size_t)W * 8, st>>>(W, denv, dsin, dcond, drowsum, wall, rowSum);
             k_env_marginal_block<<<1, kEnvThreads, mostH, st>>>(H, drowsum, rowSum, dmarg, drowProb, drowAlias, total);
             k_alias_row_block<<<H, kEnvThreads, mostW, st>>>(W, H, wall, rowSum, dcolProb, dcolAlias, dapdf, total);
