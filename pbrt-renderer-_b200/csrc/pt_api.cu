@@ -641,6 +641,7 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
     if (!ctx) return PT_E_INVALID;
     if (!d) return ctx->fail(PT_E_INVALID, "null scene");
     cudaSetDevice(ctx->device);
+    drop_earlier_error();
     cudaStreamSynchronize(ctx->stream);
     ctx->free_scene();
     if (d->num_vertices && !d->positions) return ctx->fail(PT_E_INVALID, "positions is null");
@@ -1072,6 +1073,7 @@ int pt_bsdf_eval_batch_noalloc(void *stream, const pt_material *materials, uint3
     if (loc != PT_MEM_HOST && loc != PT_MEM_DEVICE) return PT_E_INVALID;
     if (loc == PT_MEM_HOST && (n > PT_NOALLOC_MAX_QUERIES || nm > PT_NOALLOC_MAX_MATERIALS)) return PT_E_LIMIT;
     if (!n) return PT_OK;
+    drop_earlier_error();
     cudaStream_t st = (cudaStream_t)stream;
     if (loc == PT_MEM_DEVICE) {  // arrays used in place: no staging at all
         k_bsdf_eval<<<blocks_for(n), 256, 0, st>>>(materials, nm, mi, wi, wo, h, n, f, pdf);

@@ -14,6 +14,11 @@
         if (e_ != cudaSuccess) return ctx->fail(PT_E_CUDA, #call, cudaGetErrorString(e_)); \
     } while (0)
 
+// An entry point that reads cudaGetLastError() after its launches calls this
+// first: the runtime keeps the error of an earlier call on the thread (a
+// refused allocation, say, already reported by that call) until it is read.
+inline void drop_earlier_error() { (void)cudaGetLastError(); }
+
 // Device error flag bits (raised by kernels, read after a sync).
 enum : uint32_t {
     PT_DEVERR_STACK = 1u,     // traversal stack overflow

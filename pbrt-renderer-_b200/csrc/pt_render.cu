@@ -2401,6 +2401,7 @@ void pt_graph_free(pt_ctx *ctx) {
 }
 
 int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *d_comp, pt_stats *stats) {
+    drop_earlier_error();
     const uint32_t W = P->width, H = P->height;
     const uint64_t npix = (uint64_t)W * H;
     const uint64_t total = npix * P->spp;
@@ -2709,6 +2710,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
     int rc = batch_check(ctx, R, n);
     if (rc) return rc;
     cudaSetDevice(ctx->device);
+    drop_earlier_error();
     BatchState &Bt = ctx->batch;
     uint64_t total = 0;
     for (uint32_t i = 0; i < n; i++) total += (uint64_t)R[i].params.width * R[i].params.height * R[i].params.spp;
