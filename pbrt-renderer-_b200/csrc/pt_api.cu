@@ -637,10 +637,7 @@ static int upload_textures(pt_ctx *ctx, const pt_scene_desc *d) {
     return PT_OK;
 }
 
-int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
-    if (!ctx) return PT_E_INVALID;
-    if (!d) return ctx->fail(PT_E_INVALID, "null scene");
-    cudaSetDevice(ctx->device);
+static int upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
     drop_earlier_error();
     cudaStreamSynchronize(ctx->stream);
     ctx->free_scene();
@@ -964,6 +961,25 @@ int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
     ctx->clsMask = clsMask;
     ctx->hasScene = true;
     return PT_OK;
+}
+
+int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
+    if (!ctx) return PT_E_INVALID;
+    if (!d) return ctx->fail(PT_E_INVALID, "null scene");
+    cudaSetDevice(ctx->device);
+    DeviceArena &scene = ctx->sceneMem, &build = ctx->buildMem;
+    const bool kept = !scene.chunks.empty() || !build.chunks.empty();
+    scene.failed = build.failed = false;
+    int rc = upload_scene(ctx, d);
+    if (rc != PT_OK && kept && (scene.failed || build.failed)) {
+        // memory kept from the upload before, in pieces that do not fit this
+        // scene's arrays: once more with nothing kept
+        cudaStreamSynchronize(ctx->stream);
+        scene.release();
+        build.release();
+        rc = upload_scene(ctx, d);
+    }
+    return rc;
 }
 
 int pt_render(pt_ctx *ctx, const pt_render_params *p, pt_film *film, pt_stats *stats) {

@@ -941,7 +941,7 @@ int pt_cache_prepare(pt_ctx *ctx, size_t queryCap) {
     C.queryCap = 0;
     C.gen++;
     for (float4 *&p : C.q)
-        if (cudaMalloc(&p, queryCap * sizeof(float4)) != cudaSuccess)
+        if (ctx->device_alloc((void **)&p, queryCap * sizeof(float4)) != cudaSuccess)
             return ctx->fail(PT_E_NOMEM, "cache query buffers");
     C.queryCap = queryCap;
     return PT_OK;
@@ -963,7 +963,7 @@ int pt_cache_init(pt_ctx *ctx, const pt_cache_params *params) {
     if (C.params.max_train_fraction <= 0.0f || C.params.max_train_fraction > 1.0f) C.params.max_train_fraction = 0.25f;
     rc_bounds(ctx);
     cudaError_t e = cudaSuccess;
-    auto A = [&](void **p, size_t b) { if (e == cudaSuccess) e = cudaMalloc(p, b); };
+    auto A = [&](void **p, size_t b) { if (e == cudaSuccess) e = ctx->device_alloc(p, b); };
     for (float **p : {&C.w, &C.m, &C.v, &C.ema, &C.grad}) A((void **)p, kRcParams * sizeof(float));
     A((void **)&C.gradPart, (size_t)ctx->numSMs * kRcParams * sizeof(float));
     A((void **)&C.imgTrain, kRcImageBytes);

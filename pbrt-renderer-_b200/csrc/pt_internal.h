@@ -180,6 +180,7 @@ struct DeviceArena {
     struct Chunk { char *p; size_t size, used; };
     std::vector<Chunk> chunks;
     size_t minChunk;  // 0: chunks of exactly the size asked for (temporaries)
+    bool failed = false;  // an allocation has failed since this was cleared
     explicit DeviceArena(size_t minChunk_ = 0) : minChunk(minChunk_) {}
     DeviceArena(const DeviceArena &) = delete;
     DeviceArena &operator=(const DeviceArena &) = delete;
@@ -196,6 +197,7 @@ struct DeviceArena {
         const cudaError_t e = cudaMalloc((void **)&c.p, c.size);
         *out = c.p;
         if (e == cudaSuccess) chunks.push_back(c);
+        else failed = true;
         return e;
     }
     // One chunk of at least `bytes`, empty (a workspace's start).
@@ -257,8 +259,9 @@ struct pt_ctx {
     std::string err;
     DeviceArena sceneMem{(size_t)1 << 20};  // the uploaded scene's arrays
     // workspace of uploads (about 190 bytes a triangle), kept for the next one
-    // until the wave buffers have to grow: mapping and unmapping it took from 1
-    // to 200 ms per upload, whatever else the driver was doing
+    // until the wave buffers have to grow or an allocation needs it
+    // (device_alloc, pt_upload_scene): mapping and unmapping it took from 1 to
+    // 200 ms per upload, whatever else the driver was doing
     DeviceArena buildMem;
     pt::DevScene S{};
     bool hasScene = false;
@@ -285,6 +288,17 @@ struct pt_ctx {
         if (detail) { err += ": "; err += detail; }
         return code;
     }
+    // cudaMalloc; where it fails, once more without the upload workspace.  (Not
+    // during an upload, whose temporaries live there.)
+    cudaError_t device_alloc(void **p, size_t bytes) {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation && !buildMem.chunks.empty()) {
+            buildMem.release();
+            e = cudaMalloc(p, bytes);
+        }
+        if (e != cudaSuccess) *p = nullptr;
+        return e;
+    }
     template <class T>
     cudaError_t alloc_scene(T **p, size_t count) {
         return sceneMem.alloc((void **)p, count * sizeof(T) + 16);
@@ -305,7 +319,7 @@ inline int scratch(pt_ctx *ctx, size_t bytes, char **out) {
         if (ctx->scratch) cudaFree(ctx->scratch);
         ctx->scratch = nullptr;
         ctx->scratchBytes = 0;
-        cudaError_t e = cudaMalloc(&ctx->scratch, bytes);
+        cudaError_t e = ctx->device_alloc(&ctx->scratch, bytes);
         if (e != cudaSuccess) return ctx->fail(PT_E_NOMEM, "scratch", cudaGetErrorString(e));
         ctx->scratchBytes = bytes;
     }

@@ -1910,7 +1910,7 @@ static int wave_alloc(pt_ctx *ctx, size_t cap) {
     WaveBuffers &W = ctx->W;
     size_t sc = 2 * cap;
     cudaError_t e = cudaSuccess;
-    auto A = [&](void **p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
+    auto A = [&](void **p, size_t bytes) { if (e == cudaSuccess) e = ctx->device_alloc(p, bytes); };
     A((void **)&W.thr_pdf, cap * 16); A((void **)&W.lo_eta, cap * 16);
     A((void **)&W.pendA, cap * 16); A((void **)&W.pendE, cap * 16); A((void **)&W.rng, cap * 16);
     for (int k = 0; k < 2; k++) { A((void **)&W.qslot[k], cap * 4); A((void **)&W.qo[k], cap * 16); A((void **)&W.qd[k], cap * 16); }
@@ -1975,7 +1975,7 @@ int counters_alloc(pt_ctx *ctx, uint32_t depth) {
     if (W.counters) cudaFree(W.counters);
     W.counters = nullptr;
     W.counterBounces = 0;
-    cudaError_t e = cudaMalloc((void **)&W.counters, (1 + want) * kCounterWords * sizeof(uint32_t));
+    cudaError_t e = ctx->device_alloc((void **)&W.counters, (1 + want) * kCounterWords * sizeof(uint32_t));
     if (e != cudaSuccess) return ctx->fail(PT_E_NOMEM, "wave counters", cudaGetErrorString(e));
     W.counterBounces = want;
     ctx->waveGen++;
@@ -2732,10 +2732,11 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         if (Bt.slotInfo) cudaFree(Bt.slotInfo);
         Bt.slotInfo = nullptr;
         Bt.slotCap = 0;
-        if (cudaMalloc(&Bt.slotInfo, cap * sizeof(uint2)) != cudaSuccess) return ctx->fail(PT_E_NOMEM, "batch slots");
+        if (ctx->device_alloc((void **)&Bt.slotInfo, cap * sizeof(uint2)) != cudaSuccess)
+            return ctx->fail(PT_E_NOMEM, "batch slots");
         Bt.slotCap = cap;
     }
-    if (!Bt.reqs && cudaMalloc(&Bt.reqs, PT_BATCH_MAX_REQUESTS * sizeof(ReqDev)) != cudaSuccess)
+    if (!Bt.reqs && ctx->device_alloc(&Bt.reqs, PT_BATCH_MAX_REQUESTS * sizeof(ReqDev)) != cudaSuccess)
         return ctx->fail(PT_E_NOMEM, "batch request table");
     if (!gExt) {
         gExt = grid_for(ctx, (const void *)k_extend<false>);
@@ -2772,7 +2773,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
         if (Bt.films) cudaFree(Bt.films);
         Bt.films = nullptr;
         Bt.filmBytes = 0;
-        if (cudaMalloc(&Bt.films, stage) != cudaSuccess) return ctx->fail(PT_E_NOMEM, "batch film staging");
+        if (ctx->device_alloc(&Bt.films, stage) != cudaSuccess) return ctx->fail(PT_E_NOMEM, "batch film staging");
         Bt.filmBytes = stage;
     }
     std::vector<ReqDev> hostReqs(n);
@@ -2955,7 +2956,7 @@ extern "C" int pt_batch_autotune(pt_ctx *ctx, const pt_request *requests, uint32
         maxPix = std::max<uint64_t>(maxPix, (uint64_t)requests[i].params.width * requests[i].params.height);
     }
     float *film = nullptr;
-    if (cudaMalloc(&film, maxPix * 32) != cudaSuccess) return ctx->fail(PT_E_NOMEM, "tuning film");
+    if (ctx->device_alloc((void **)&film, maxPix * 32) != cudaSuccess) return ctx->fail(PT_E_NOMEM, "tuning film");
     // candidates: wave sizes from the whole batch down to 2^22 paths, full and half traversal grids
     std::vector<size_t> waves;
     for (uint64_t w = std::min<uint64_t>(total, kMaxWavePaths);; w >>= 1) {
