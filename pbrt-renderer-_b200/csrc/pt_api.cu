@@ -763,12 +763,15 @@ static int upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
             ctx->sceneMax[k] = hi[k];
         }
     }
-    float *dpos, *dnrm, *duv, *dtan, *dcdf;
+    float *duv, *dtan, *dcdf;
     uint32_t *didx, *dmft, *demit;
+    float4 *dpos4, *dnrm4;
+    uint4 *dtidx;
+    uint8_t *dtcls;
     pt_material *dmats;
     cudaStream_t st = ctx->stream;
-    PT_CUDA(ctx->alloc_scene(&dpos, 3 * nv + 3));
-    PT_CUDA(ctx->alloc_scene(&dnrm, 3 * nv + 3));
+    PT_CUDA(ctx->alloc_scene(&dpos4, nv + 1));
+    PT_CUDA(ctx->alloc_scene(&dnrm4, nv + 1));
     PT_CUDA(ctx->alloc_scene(&duv, 2 * nv + 2));
     PT_CUDA(ctx->alloc_scene(&dtan, 3 * nv + 3));
     PT_CUDA(ctx->alloc_scene(&didx, (size_t)d->num_indices + 1));
@@ -776,8 +779,20 @@ static int upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
     PT_CUDA(ctx->alloc_scene(&dmft, meshFirstTri.size()));
     PT_CUDA(ctx->alloc_scene(&dcdf, all.size() + 1));
     PT_CUDA(ctx->alloc_scene(&demit, (size_t)ne + 1));
+    PT_CUDA(ctx->alloc_scene(&dtidx, (size_t)numTris + 1));
+    PT_CUDA(ctx->alloc_scene(&dtcls, (size_t)numTris + 1));
+    // what is only read to make those records, in the workspace (the build
+    // begins it anew when they are made)
+    float *dpos, *dnrm;
     uint32_t *dmcls;
-    PT_CUDA(ctx->alloc_scene(&dmcls, meshClass.size()));
+    {
+        DeviceArena &tmp = ctx->buildMem;
+        const size_t need = 2 * (3 * nv * 4 + 256) + meshClass.size() * 4 + 256;
+        PT_CUDA(tmp.begin(std::max(need, pt_bvh_workspace(ctx, numTris))));
+        PT_CUDA(tmp.alloc((void **)&dpos, 3 * nv * 4));
+        PT_CUDA(tmp.alloc((void **)&dnrm, 3 * nv * 4));
+        PT_CUDA(tmp.alloc((void **)&dmcls, meshClass.size() * 4));
+    }
     auto h2d = [&](void *dst, const void *src, size_t bytes) -> int {
         if (!bytes) return PT_OK;
         cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
@@ -786,7 +801,7 @@ static int upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
     int rc;
     if ((rc = h2d(dpos, d->positions, 3 * nv * 4))) return rc;
     if (d->normals) { if ((rc = h2d(dnrm, d->normals, 3 * nv * 4))) return rc; }
-    else PT_CUDA(cudaMemsetAsync(dnrm, 0, 3 * nv * 4 + 12, st));
+    else PT_CUDA(cudaMemsetAsync(dnrm, 0, 3 * nv * 4, st));
     if (d->texcoords) { if ((rc = h2d(duv, d->texcoords, 2 * nv * 4))) return rc; }
     else PT_CUDA(cudaMemsetAsync(duv, 0, 2 * nv * 4 + 8, st));
     if (d->tangents) { if ((rc = h2d(dtan, d->tangents, 3 * nv * 4))) return rc; }
@@ -809,17 +824,10 @@ static int upload_scene(pt_ctx *ctx, const pt_scene_desc *d) {
         S.mediaTrDeferred = 0u;
         if (S.mediaWavefront) clsMask |= 1u << CLS_MEDIUM;
     }
-    S.pos = dpos; S.uv = duv; S.tan = dtan; S.idx = didx;
+    S.uv = duv; S.tan = dtan; S.idx = didx;
     S.mats = dmats; S.numMeshes = d->num_meshes; S.meshFirstTri = dmft;
     S.emitterCdf = dcdf; S.emitterList = demit; S.emitterCount = ne;
     S.hasGlass = hasGlass ? 1u : 0u;
-    float4 *dpos4, *dnrm4;
-    uint4 *dtidx;
-    uint8_t *dtcls;
-    PT_CUDA(ctx->alloc_scene(&dpos4, nv + 1));
-    PT_CUDA(ctx->alloc_scene(&dnrm4, nv + 1));
-    PT_CUDA(ctx->alloc_scene(&dtidx, (size_t)numTris + 1));
-    PT_CUDA(ctx->alloc_scene(&dtcls, (size_t)numTris + 1));
     S.pos4 = dpos4; S.nrm4 = dnrm4; S.triIdx = dtidx; S.triClass = dtcls;
     if (nv) k_pack_vertices<<<(unsigned)std::min<size_t>((nv + 255) / 256, 4096), 256, 0, st>>>(nv, dpos, dnrm, dpos4, dnrm4);
     if (numTris) {  // every index within its mesh's vertices, before a kernel follows one

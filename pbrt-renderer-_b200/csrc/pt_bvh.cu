@@ -122,7 +122,7 @@ __device__ __forceinline__ uint32_t expand_bits(uint32_t v) {
 // Triangle bounds, mesh of each triangle and centroid (exact float ops).
 __global__ void k_tri_bounds(uint32_t n, const uint32_t *__restrict__ meshFirstTri, uint32_t numMeshes,
                              const pt_material *__restrict__ mats, const uint32_t *__restrict__ idx,
-                             const float *__restrict__ pos, uint32_t *triMesh, float4 *lo, float4 *hi,
+                             const float4 *__restrict__ pos, uint32_t *triMesh, float4 *lo, float4 *hi,
                              float4 *cen) {
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
@@ -133,9 +133,9 @@ __global__ void k_tri_bounds(uint32_t n, const uint32_t *__restrict__ meshFirstT
     }
     const pt_material &m = mats[a];
     uint32_t base = m.indexOffset + 3u * (g - meshFirstTri[a]);
-    float3 p0 = ld3(pos, m.vertexOffset + idx[base]);
-    float3 p1 = ld3(pos, m.vertexOffset + idx[base + 1]);
-    float3 p2 = ld3(pos, m.vertexOffset + idx[base + 2]);
+    float3 p0 = ld4(pos, m.vertexOffset + idx[base]);
+    float3 p1 = ld4(pos, m.vertexOffset + idx[base + 1]);
+    float3 p2 = ld4(pos, m.vertexOffset + idx[base + 2]);
     float3 l = vmin(p0, vmin(p1, p2)), h = vmax(p0, vmax(p1, p2));
     triMesh[g] = a;
     lo[g] = make_float4(l.x, l.y, l.z, 0.0f);
@@ -607,7 +607,7 @@ struct CollapseIn {
     const uint32_t *triMesh, *meshFirstTri;
     const pt_material *mats;
     const uint32_t *idx;
-    const float *pos;
+    const float4 *pos;
     BVH8Node *nodes;
     float4 *tri;
     uint32_t *counters;  // [0] wide nodes allocated, [1] triangles written, [2] next queue size, [3] error
@@ -770,9 +770,9 @@ __global__ void k_collapse(CollapseIn C, const int2 *__restrict__ qin, uint32_t 
                 uint32_t mesh = C.triMesh[g];
                 const pt_material &m = C.mats[mesh];
                 uint32_t base = m.indexOffset + 3u * (g - C.meshFirstTri[mesh]);
-                float3 p0 = ld3(C.pos, m.vertexOffset + C.idx[base]);
-                float3 p1 = ld3(C.pos, m.vertexOffset + C.idx[base + 1]);
-                float3 p2 = ld3(C.pos, m.vertexOffset + C.idx[base + 2]);
+                float3 p0 = ld4(C.pos, m.vertexOffset + C.idx[base]);
+                float3 p1 = ld4(C.pos, m.vertexOffset + C.idx[base + 1]);
+                float3 p2 = ld4(C.pos, m.vertexOffset + C.idx[base + 2]);
                 float3 e1 = p1 - p0, e2 = p2 - p0;
                 float4 *t = C.tri + 3u * (triBase + toff + k);
                 t[0] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(g));
@@ -799,6 +799,17 @@ __global__ void k_collapse(CollapseIn C, const int2 *__restrict__ qin, uint32_t 
 
 using namespace pt;
 
+// Which collapse is tried first (pt_build_bvh_device, at the collapse).
+static bool plan_first(const pt_ctx *ctx, uint32_t n) {
+    int l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
+    return ctx->dbgWidePlan || (uint64_t)n * 71u > (uint64_t)(l2 > 0 ? l2 : 126 << 20);
+}
+
+size_t pt_bvh_workspace(const pt_ctx *ctx, uint32_t n) {
+    return n ? (size_t)n * (plan_first(ctx, n) ? 230 : 188) + ((size_t)n / kRsTile + 1) * 1024 + 16384 : 0;
+}
+
 // Exact floating-point bounds are needed by the element subtraction in
 // k_collapse's e1/e2: they use the same IEEE subtraction as the oracle.
 int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n) {
@@ -820,12 +831,9 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
     // temporaries, in the context's build workspace
     DeviceArena &tmp = ctx->buildMem;
     auto cleanup = [&]() { tmp.rewind(); };
-    // (planFirst: which collapse is tried first, below)
-    int l2 = 0;
-    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
-    const bool planFirst = ctx->dbgWidePlan || (uint64_t)n * 71u > (uint64_t)(l2 > 0 ? l2 : 126 << 20);
+    const bool planFirst = plan_first(ctx, n);
     {
-        const cudaError_t e = tmp.begin((size_t)n * (planFirst ? 230 : 188) + ((size_t)n / kRsTile + 1) * 1024 + 16384);
+        const cudaError_t e = tmp.begin(pt_bvh_workspace(ctx, n));
         if (e != cudaSuccess) return ctx->fail(PT_E_NOMEM, "bvh temp", cudaGetErrorString(e));
     }
 #define TA(p, bytes)                                                                   \
@@ -846,7 +854,7 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
     TA(qa, (size_t)n * 8); TA(qb, (size_t)n * 8);
     const int B = 256;
     uint32_t G = (n + B - 1) / B;
-    k_tri_bounds<<<G, B, 0, st>>>(n, d_meshFirstTri, S.numMeshes, S.mats, S.idx, S.pos, triMesh, tlo, thi, cen);
+    k_tri_bounds<<<G, B, 0, st>>>(n, d_meshFirstTri, S.numMeshes, S.mats, S.idx, S.pos4, triMesh, tlo, thi, cen);
     uint32_t binit[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
     cudaMemcpyAsync(bounds, binit, sizeof(binit), cudaMemcpyHostToDevice, st);
     k_centroid_bounds<<<min(G, 1024u), B, 0, st>>>(n, cen, bounds);
@@ -944,7 +952,7 @@ int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t n)
             planW = planWide;
         }
         CollapseIn C{(int)n, radix ? children : tch, cnt, maxWide, leafLo, leafHi, intLo, intHi, idsS, triMesh,
-                     d_meshFirstTri, S.mats, S.idx, S.pos, nodes, tri, counters, plan, planW};
+                     d_meshFirstTri, S.mats, S.idx, S.pos4, nodes, tri, counters, plan, planW};
         int2 root = make_int2(n > 1 ? 0 : ~0, 0);
         cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, st);
         uint32_t cinit[4] = {1u, 0u, 0u, 0u};

@@ -45,7 +45,7 @@ struct DevScene {
     const pt_material *mats;
     uint32_t numMeshes;
     uint32_t hasGlass;            // any mirror/dielectric mesh (non-opaque for shadow rays)
-    const float *pos, *uv, *tan;
+    const float *uv, *tan;
     const uint32_t *idx;
     // for shading: vertex positions and normals as 16-byte records, and per
     // global triangle id its three vertices and mesh in one, and its shading

@@ -378,6 +378,7 @@ struct Staging {
 // pt_bvh.cu: builds S.tri / S.nodes / S.triMesh / S.meshFirstTri and the
 // parity exports on the device from the uploaded geometry.
 int pt_build_bvh_device(pt_ctx *ctx, const uint32_t *d_meshFirstTri, uint32_t numTris);
+size_t pt_bvh_workspace(const pt_ctx *ctx, uint32_t numTris);  // bytes of buildMem that takes
 // pt_render.cu
 int pt_render_impl(pt_ctx *ctx, const pt_render_params *p, float *d_sum, float *d_comp, pt_stats *stats);
 int pt_wave_free(pt_ctx *ctx);

@@ -80,3 +80,28 @@ def test_a_larger_scene_takes_the_previous_scenes_memory(pt, scenes):
             assert np.array_equal(film, want)
         finally:
             ctx.close()
+
+
+def test_a_vertex_takes_52_bytes(pt):
+    """Resident after an upload and a render: 16-byte positions and normals,
+    texture coordinates and tangents, and not also the arrays that the records
+    were made from.  (48 MB beside them: wave buffers and rounding.)"""
+    import torch
+
+    n = 8_000_000
+    m = pt.make_material(pt.PT_MAT_DIFFUSE)
+    m.vertexCount, m.indexCount = 3, 3
+    cam = pt.pt_camera()
+    P = pt.render_params(64, 64, 1, cam, max_depth=2)
+    for nv in (3, n):  # the first: the kernels' own memory
+        sc = pt.Scene(np.eye(3, dtype=np.float32)[np.arange(nv) % 3], np.array([0, 1, 2]), [m],
+                      normals=np.ones((nv, 3), np.float32))
+        free = torch.cuda.mem_get_info()[0]
+        ctx = pt.Context(0)
+        try:
+            ctx.upload(sc)
+            ctx.render(P)  # its buffers grow: the workspace is given back
+            used = free - torch.cuda.mem_get_info()[0]
+        finally:
+            ctx.close()
+    assert 52 * n <= used <= 60 * n + 48 * MB
