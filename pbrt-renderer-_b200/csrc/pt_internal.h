@@ -392,6 +392,7 @@ cudaError_t rc_enqueue_targets(pt_ctx *ctx, cudaStream_t st, float4 *lo_eta, uin
                                const float4 *pendE, uint32_t keyRange);
 // one training step s of kRcStepsPerCall: the network kernel (adam = false) or its Adam update (adam = true)
 cudaError_t rc_enqueue_train(pt_ctx *ctx, cudaStream_t st, uint32_t s, bool adam);
+constexpr uint32_t kRcTargetLaunches = 5;  // kernels of rc_enqueue_targets
 constexpr uint32_t kRcStepsPerCall = 4;  // Adam steps per cached render call, on interleaved quarters of its records
 void pt_graph_free(pt_ctx *ctx);
 void pt_branch_free(pt_ctx *ctx, int k);

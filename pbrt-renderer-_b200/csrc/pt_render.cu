@@ -2020,10 +2020,9 @@ struct Enqueue {
     cudaStream_t st;
     bool timing;
     std::vector<Mark> marks;
-    uint64_t launches = 0;
+    uint64_t launches = 0;  // kernels, counted where they are issued
     const ForkJoin *fj = nullptr;  // set in captures: issue independent kernels as parallel branches
     void begin(int stage) {
-        launches++;
         if (!timing) return;
         Mark m{stage, nullptr, nullptr};
         cudaEventCreate(&m.a);
@@ -2053,11 +2052,30 @@ inline Shape queue_shape(int grid, uint64_t n, uint64_t paths, int numSMs) {
     const unsigned block = paths <= (uint64_t)numSMs * 1024u ? 64u : (unsigned)kBlock;
     return {(unsigned)std::min<uint64_t>((n + block - 1) / block, (uint64_t)grid * (kBlock / block)), block};
 }
-// Kernels per bounce of a wave (launch counts).
-inline uint32_t bounce_launches(const pt_ctx *ctx, const WaveArgs &A) {
-    if ((ctx->S.numVols > 0 && !A.S.mediaWavefront) || ctx->S.hasSubsurface) return 2 + A.flightPass;
-    return 2 + (uint32_t)__builtin_popcount(ctx->clsMask | (A.S.mediaWavefront ? 1u << CLS_MEDIUM : 0u)) +
-           2 * A.flightPass + A.ratioPass;
+// The forms of a traversal kernel that bounce b launches over a queue of at
+// most `most` rays: `one` with a lane per ray, `eight` with 8 lanes.  The
+// queue's length decides on the device, so both are launched where it is not
+// known here.  `eight` is left out where the queue is hardly that short yet (a
+// quarter of the paths going on at each bounce), and `one` then takes queues
+// of any length.  (As parallel nodes they saved no time, and the wider graph
+// took 3 ms more to instantiate.)
+struct Forms { bool one, eight; };
+inline Forms forms(const WaveArgs &A, uint32_t b, uint64_t most) {
+    const bool eight = A.coopMax && (b > 15u || (A.waveCount >> (2u * b)) <= A.coopMax);
+    return {!eight || most > A.coopMax, eight};
+}
+// Kernels of bounce b of a wave.
+inline uint32_t bounce_launches(const pt_ctx *ctx, const WaveArgs &A, uint32_t b) {
+    auto count = [&](uint64_t most) {
+        const Forms f = forms(A, b, most);
+        return (f.one ? 1u : 0u) + (f.eight ? 1u : 0u);
+    };
+    if ((ctx->S.numVols > 0 && !A.S.mediaWavefront) || ctx->S.hasSubsurface)
+        return count(A.waveCount) + A.flightPass + 1u;
+    const uint32_t extend = A.flightPass ? count(A.waveCount) + 2u : A.S.mediaWavefront ? 1u : count(A.waveCount);
+    const uint32_t shadow = (A.S.mediaTrDeferred ? 1u : count(2ull * A.waveCount)) + A.ratioPass;
+    return extend + shadow +
+           (uint32_t)__builtin_popcount(ctx->clsMask | (A.S.mediaWavefront ? 1u << CLS_MEDIUM : 0u));
 }
 
 cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t first, uint32_t depth,
@@ -2080,7 +2098,9 @@ bool enqueue_rest_conditional(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32
         cudaGetLastError();
         return false;
     }
-    k_tail_close<<<1, 1, 0, E.st>>>(A, h, (depth - first) * bounce_launches(ctx, A));
+    uint32_t rest = 0;
+    for (uint32_t b = first; b < depth; b++) rest += bounce_launches(ctx, A, b);
+    k_tail_close<<<1, 1, 0, E.st>>>(A, h, rest);
     auto chk = [&](cudaError_t e) {
         if (err == cudaSuccess && e != cudaSuccess) err = e;
     };
@@ -2135,6 +2155,7 @@ cudaError_t enqueue_paths(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t d
     A.qslotOut = B.qslot[0]; A.qoOut = B.qo[0]; A.qdOut = B.qd[0]; A.cntOut = B.counters + kCounterWords;
     E.begin(STG_RAYGEN);
     k_raygen<<<(A.waveCount + kBlock - 1) / kBlock, kBlock, 0, E.st>>>(A);
+    E.launches++;
     E.end();
     const cudaError_t e = enqueue_bounces(ctx, E, A, 0, depth, G, true);
     return err != cudaSuccess ? err : e;
@@ -2156,20 +2177,13 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
         if (shadowOpen) chk(cudaStreamWaitEvent(st, fj->joinEv[0], 0));
         shadowOpen = false;
     };
-    // The two forms of a traversal kernel over a queue of at most `most` rays,
-    // `one` a lane per ray and `eight` 8 lanes: the queue's length decides on
-    // the device, so both are launched where it is not known here.  `eight` is
-    // left out where the queue is hardly that short yet (a quarter of the paths
-    // going on at each bounce), and `one` then takes queues of any length.
-    // (As parallel nodes they saved no time, and the wider graph took 3 ms more
-    // to instantiate.)
     const unsigned coopGrid = (unsigned)std::min<uint64_t>(2ull * A.waveCount, kCoopMax) * 8u / kCoopBlock + 1u;
     const uint32_t coopMax = A.coopMax;
     auto both = [&](uint64_t most, auto one, auto eight) {
-        const bool useEight = coopMax && (A.bounce > 15u || (A.waveCount >> (2u * A.bounce)) <= coopMax);
-        A.coopMax = useEight ? coopMax : 0u;
-        if (most > A.coopMax) one();
-        if (useEight) eight();
+        const Forms f = forms(A, A.bounce, most);
+        A.coopMax = f.eight ? coopMax : 0u;
+        if (f.one) one();
+        if (f.eight) eight();
         A.coopMax = coopMax;
     };
     for (uint32_t b = first; b < depth; b++) {
@@ -2196,6 +2210,7 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
                 k_tail<false><<<G.tail, kBlock, 0, st>>>(A);
                 if (A.coopTailMax) k_tail8<<<kCoopTailMax * 8u / kCoopBlock, kCoopBlock, 0, st>>>(A);
             }
+            E.launches += 2u + (!inl && A.coopTailMax ? 1u : 0u);
             if (fj) {
                 if (enqueue_rest_conditional(ctx, E, A, b, depth, G, err)) return err;
             }
@@ -2208,6 +2223,7 @@ cudaError_t enqueue_bounces(const pt_ctx *ctx, Enqueue &E, WaveArgs &A, uint32_t
                 if (err == cudaSuccess && left == 0u) return err;
             }
         }
+        E.launches += bounce_launches(ctx, A, b);
         if (inl) {
             const Shape x = shape(G.ext, A.waveCount), h = shape(G.shadeI, A.waveCount);
             E.begin(STG_EXTEND);
@@ -2332,11 +2348,13 @@ cudaError_t enqueue_render(const pt_ctx *ctx, Enqueue &E, WaveArgs A, const pt_r
             // the cache value at a training record's vertex
             E.begin(STG_CACHE_INFER);
             chk(rc_enqueue_resolve(const_cast<pt_ctx *>(ctx), st, A.lo_eta));
+            E.launches++;
             E.end();
             // training targets from the suffixes, then the training paths' image
             // values (prefix + throughput x cache); counts the wave's queries
             E.begin(STG_CACHE);
             chk(rc_enqueue_targets(const_cast<pt_ctx *>(ctx), st, A.lo_eta, A.rng, A.pendA, A.pendE, A.recKeyRange));
+            E.launches += kRcTargetLaunches;
             E.end();
         }
         uint32_t cover = (uint32_t)npix;  // k_film: one thread per pixel position
@@ -2348,6 +2366,7 @@ cudaError_t enqueue_render(const pt_ctx *ctx, Enqueue &E, WaveArgs A, const pt_r
         }
         E.begin(STG_FILM);
         k_film<<<(cover + kBlock - 1) / kBlock, kBlock, 0, st>>>(A, (float4 *)d_sum, (float4 *)d_comp);
+        E.launches++;
         E.end();
         chk(cudaGetLastError());  // launch-configuration errors of this wave
     }
@@ -2358,6 +2377,7 @@ cudaError_t enqueue_render(const pt_ctx *ctx, Enqueue &E, WaveArgs A, const pt_r
             E.end();
             E.begin(STG_CACHE);
             chk(rc_enqueue_train(const_cast<pt_ctx *>(ctx), st, step, true));
+            E.launches += 2;  // with the gradient's
             E.end();
         }
     }
@@ -2481,9 +2501,12 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     for (float4 *&q : A.cq) q = nullptr;
     for (float4 *&r : A.cr) r = nullptr;
     A.cqCount = A.crCount = nullptr;
+    uint64_t launches = 1;  // the sample offset's
     if (A.cacheOn) {
+        const bool first = ctx->cache.firstCall;
         if ((rc = rc_render_setup(ctx, B.cap, total))) return rc;
         const RadianceCache &C = ctx->cache;
+        if (first && !C.firstCall) launches++;  // the training chance's
         A.roughThr = C.params.rough_threshold;
         A.unbiasedEvery = C.params.unbiased_every;
         A.recCap = (uint32_t)C.recCap;
@@ -2537,7 +2560,6 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     cudaEventRecord(ev[0], st);
     k_set_u32<<<1, 1, 0, st>>>(ctx->d_err + 1, P->sample_offset);
     Enqueue E{st, timing, {}, 0};
-    uint64_t launches = 1;
     if (useGraph) {
         PT_CUDA(cudaGraphLaunch(ctx->graph.exec, st));
         launches += ctx->graph.launches;
@@ -2690,6 +2712,7 @@ cudaError_t enqueue_batch(const pt_ctx *ctx, Enqueue &E, WaveArgs A, const Batch
         for (uint32_t j : pl.waveReqs[w]) {
             E.begin(STG_FILM);
             k_film_req<<<(hostReqs[j].npix + kBlock - 1) / kBlock, kBlock, 0, st>>>(A, j);
+            E.launches++;
             E.end();
             chk(cudaGetLastError(), "film launch");
         }
