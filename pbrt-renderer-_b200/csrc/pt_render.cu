@@ -1948,6 +1948,29 @@ const Kernel *const kShadeClsX = ShadeTable<true>::k;
 int gExt = 0, gExtC = 0, gExtM = 0, gShadeI = 0, gShadow = 0, gShadowM = 0, gCls[CLS_N], gClsX[CLS_N];
 int gTail = 0, gTailI = 0, gFlight = 0, gRatio = 0;
 
+// Resident grids of the kernels, worked out by the process's first render while
+// the others wait for it: contexts may be on threads of their own.
+void grids_init(pt_ctx *ctx) {
+    static const bool once = [ctx] {
+        gExt = grid_for(ctx, (const void *)k_extend<false>);
+        gExtC = grid_for(ctx, (const void *)k_extend<true>);
+        gExtM = grid_for(ctx, (const void *)k_extend_media);
+        gShadeI = grid_for(ctx, (const void *)k_shade<true, CLS_ANY>);
+        gShadow = grid_for(ctx, (const void *)k_shadow);
+        gShadowM = grid_for(ctx, (const void *)k_shadow_media);
+        for (int c = 0; c < CLS_N; c++) {
+            gCls[c] = grid_for(ctx, (const void *)kShadeCls[c]);
+            gClsX[c] = grid_for(ctx, (const void *)kShadeClsX[c]);
+        }
+        gTail = grid_for(ctx, (const void *)k_tail<false>);
+        gTailI = grid_for(ctx, (const void *)k_tail<true>);
+        gFlight = grid_for(ctx, (const void *)k_flight);
+        gRatio = grid_for(ctx, (const void *)k_ratio);
+        return true;
+    }();
+    (void)once;
+}
+
 // STG_CACHE_INFER / STG_CACHE_TRAIN: the cache's network kernels, reported
 // in ms_cache with the rest of the cache's work and on their own in the
 // cache statistics
@@ -2452,22 +2475,7 @@ int pt_render_impl(pt_ctx *ctx, const pt_render_params *P, float *d_sum, float *
     if (rc) return rc;
     cudaStream_t st = ctx->stream;
     WaveBuffers &B = ctx->W;
-    if (!gExt) {
-        gExt = grid_for(ctx, (const void *)k_extend<false>);
-        gExtC = grid_for(ctx, (const void *)k_extend<true>);
-        gExtM = grid_for(ctx, (const void *)k_extend_media);
-        gShadeI = grid_for(ctx, (const void *)k_shade<true, CLS_ANY>);
-        gShadow = grid_for(ctx, (const void *)k_shadow);
-        gShadowM = grid_for(ctx, (const void *)k_shadow_media);
-        for (int c = 0; c < CLS_N; c++) {
-            gCls[c] = grid_for(ctx, (const void *)kShadeCls[c]);
-            gClsX[c] = grid_for(ctx, (const void *)kShadeClsX[c]);
-        }
-        gTail = grid_for(ctx, (const void *)k_tail<false>);
-        gTailI = grid_for(ctx, (const void *)k_tail<true>);
-        gFlight = grid_for(ctx, (const void *)k_flight);
-        gRatio = grid_for(ctx, (const void *)k_ratio);
-    }
+    grids_init(ctx);
     WaveArgs A;
     A.S = ctx->S;
     A.width = W; A.height = H; A.npix = (uint32_t)npix;
@@ -2761,22 +2769,7 @@ int render_batch(pt_ctx *ctx, const pt_request *R, uint32_t n, float *request_ms
     }
     if (!Bt.reqs && ctx->device_alloc(&Bt.reqs, PT_BATCH_MAX_REQUESTS * sizeof(ReqDev)) != cudaSuccess)
         return ctx->fail(PT_E_NOMEM, "batch request table");
-    if (!gExt) {
-        gExt = grid_for(ctx, (const void *)k_extend<false>);
-        gExtC = grid_for(ctx, (const void *)k_extend<true>);
-        gExtM = grid_for(ctx, (const void *)k_extend_media);
-        gShadeI = grid_for(ctx, (const void *)k_shade<true, CLS_ANY>);
-        gShadow = grid_for(ctx, (const void *)k_shadow);
-        gShadowM = grid_for(ctx, (const void *)k_shadow_media);
-        for (int c = 0; c < CLS_N; c++) {
-            gCls[c] = grid_for(ctx, (const void *)kShadeCls[c]);
-            gClsX[c] = grid_for(ctx, (const void *)kShadeClsX[c]);
-        }
-        gTail = grid_for(ctx, (const void *)k_tail<false>);
-        gTailI = grid_for(ctx, (const void *)k_tail<true>);
-        gFlight = grid_for(ctx, (const void *)k_flight);
-        gRatio = grid_for(ctx, (const void *)k_ratio);
-    }
+    grids_init(ctx);
     if (gridScale <= 0.0f) gridScale = (Bt.tunedWave && Bt.tunedSceneGen == ctx->sceneGen) ? Bt.tunedGrid : 1.0f;
     auto sc = [&](int g) { return std::max(ctx->numSMs, (int)((float)g * gridScale)); };
     int clsG[CLS_N], clsGX[CLS_N];
