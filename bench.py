@@ -142,12 +142,13 @@ def measured_peaks():
 
 
 # k_extend DRAM traffic per extension ray (dram__bytes_read.sum + dram__bytes_write.sum
-# from one ncu capture of this workload at 8 spp, the smallest case in the
-# grouped path order (groups of 8 samples): 383.3 MB over the 7,372,800
-# camera rays of bounce 0; the full frame's groups of 32 are more coherent,
-# so this is an upper bound for it).  The scene is L2-resident and the
-# queues stream once, so traffic scales with the rays a launch processes.
-EXTEND_DRAM_BYTES_PER_RAY = {"disney_envmap": 52.0}
+# from one ncu capture of this workload at 8 spp, a case in groups of 8
+# samples: 381.6 MB over the 7,372,800 camera rays of bounce 0; the full
+# frame's groups of 32 are more coherent, so this is an upper bound for it).
+# The scene is L2-resident and the queues stream once, so traffic scales with
+# the rays a launch processes.
+EXTEND_DRAM_BYTES_PER_RAY = {"disney_envmap": 51.8}
+TAIL_BOUNCE = 4  # the bounce at which the tail kernel may take over (PT_TAIL_BOUNCE)
 
 
 REF_SPP = 4096        # reference image: plain path tracing, samples [0, 4096)
@@ -783,7 +784,8 @@ def main():
     sh = sum(s.shadow_rays for s in stats)
     stage_ms = {k: sum(getattr(s, "ms_" + k) for s in tstats)
                 for k in ("raygen", "extend", "shade", "shadow", "tail", "film")}
-    launches = {"extend": sum(s.bounces for s in tstats)}
+    # closest-hit launches: where the tail kernel took a frame's paths, the bounces after it do not run
+    launches = {"extend": sum(TAIL_BOUNCE * s.waves if s.tail_extension_rays else s.bounces for s in tstats)}
     # k_extend's own rays (the tail kernel traces the last bounces' rays itself)
     ext_k = sum(s.extension_rays - s.tail_extension_rays for s in tstats)
     peak, peak_src = measured_peaks()

@@ -57,8 +57,10 @@ extern "C" {
  * `subsurface`, g in `anisotropic` and its tint in sheen/sheenTint/clearcoat
  * (src/cpu/subsurface.cpp:69-90).
  * The caller fills type, colours, parameters, isEmitter/radiance and the
- * index/vertex ranges; pt_upload_scene fills surfaceArea, emitterCdfOffset
- * and emitterSelectionProb the way src/gpu/DXRApp_Scene.cpp:172-299 does.
+ * index/vertex ranges; pt_upload_scene sets surfaceArea, emitterCdfOffset and
+ * emitterSelectionProb in its own copy, for emitters the way
+ * src/gpu/DXRApp_Scene.cpp:172-299 does and to 0 for others, whose values
+ * nothing reads.
  */
 typedef struct pt_material {
     uint32_t type;
@@ -222,7 +224,7 @@ typedef struct pt_stats {
     uint64_t extension_rays;
     uint64_t shadow_rays;
     uint64_t waves;
-    uint64_t bounces;  /* wavefront iterations launched (closest-hit kernel launches) */
+    uint64_t bounces;  /* bounces of all waves; those after the tail kernel (below) run only where it left paths */
     uint64_t launches; /* kernels this call launched */
     float ms_total;    /* device time of the render, CUDA events on the context's stream */
     /* per stage, with PT_RENDER_STAGE_TIMING (0 otherwise): */
@@ -283,7 +285,9 @@ int pt_abi_version(void);
  * + BuildEnvmapDistribution (src/gpu/DXRApp_Scene.cpp:37-493,
  * src/gpu/DXRApp_Textures.cpp:281-389): copies the scene, builds the LBVH
  * and its 8-wide compressed form, the emitter CDFs, the envmap CDFs and
- * alias table, and the volume majorant grids on the device. */
+ * alias table, and the volume majorant grids on the device.  The context keeps
+ * the upload's workspace (about 190 bytes a triangle) for the next upload, until
+ * wave buffers grow or an allocation of this context needs the memory. */
 int pt_upload_scene(pt_ctx *ctx, const pt_scene_desc *scene);
 
 /* ---- render ---------------------------------------------------------------

@@ -439,9 +439,8 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSm) k_trace_shadow
     tr[3 * i] = t.x; tr[3 * i + 1] = t.y; tr[3 * i + 2] = t.z;
 }
 
-// The same with 8 lanes per ray, for queries that fit the GPU at once so
-// (kTraceCoopMax); occlusion only without glass.
-constexpr size_t kTraceCoopMax = 148u * 32u * 4u;
+// The same with 8 lanes per ray, for queries of up to kCoopMax rays; occlusion
+// only without glass.
 __global__ void __launch_bounds__(kTraceBlock) k_trace_closest8(DevScene S, const float *rays, size_t n, pt_hit *out,
                                                                 uint32_t *err) {
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
@@ -1275,7 +1274,7 @@ int pt_trace_closest(pt_ctx *ctx, const float *rays, size_t n, pt_hit *out, uint
     int rc = s.setup();
     if (rc) return rc;
     cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
-    if (n <= kTraceCoopMax)
+    if (n <= kCoopMax)
         k_trace_closest8<<<blocks_for(8 * n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(ctx->S, (float *)s.dev(0), n,
                                                                                      (pt_hit *)s.dev(1), ctx->d_err);
     else
@@ -1301,7 +1300,7 @@ int pt_trace_shadow(pt_ctx *ctx, const float *rays, size_t n, uint32_t *occ, flo
     int rc = s.setup();
     if (rc) return rc;
     cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
-    if (n <= kTraceCoopMax && !ctx->S.hasGlass)
+    if (n <= kCoopMax && !ctx->S.hasGlass)
         k_trace_shadow8<<<blocks_for(8 * n, kTraceBlock), kTraceBlock, 0, ctx->stream>>>(
             ctx->S, (float *)s.dev(0), n, (uint32_t *)s.dev(1), (float *)s.dev(2), ctx->d_err);
     else

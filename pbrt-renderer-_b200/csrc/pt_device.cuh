@@ -987,6 +987,9 @@ __device__ __forceinline__ bool trace_shadow(const DevScene &S, float3 o, float3
 // triangles 8 at a time; everything else is the same in all lanes.  Boxes,
 // their order and each triangle's arithmetic are the one-lane form's, so the
 // results are its bits.  All 8 lanes of a group call these together.
+// kCoopMax: the rays that are resident at once so (32 warps of 4 rays on each
+// of 148 SMs); queues and queries of at most that many take this form.
+constexpr uint32_t kCoopMax = 148u * 32u * 4u;
 struct Group8 {
     uint32_t mask, shift, j;
 };

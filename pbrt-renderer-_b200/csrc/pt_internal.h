@@ -250,7 +250,7 @@ struct pt_ctx {
     // branches of a captured render (ForkJoin in pt_render.cu): streams and
     // events that take part in captures only; [1]: of a conditional node's
     // body, which is a capture of its own on bodyStream
-    // (one branch: with three a 64 x 64 room's call took 0.34 ms instead of 0.35,
+    // (one branch: with six a 64 x 64 room's call took 0.34 ms instead of 0.35,
     // but the wider graph of a new context's first call 1 ms more)
     static constexpr int kBranches = 1;
     cudaStream_t branch[2][kBranches] = {}, bodyStream = nullptr;

@@ -706,12 +706,10 @@ __global__ void __launch_bounds__(kBlock, kTraversalBlocksPerSm) k_ratio(WaveArg
     }
 }
 // ---- short queues: 8 lanes per ray -------------------------------------------------
-// Launched beside k_extend / k_shadow; the queue's length decides on the
-// device which of the two does the work.  kCoopMax: the rays that are
-// resident at once with 8 lanes each (32 warps of 4 rays on 148 SMs).  64 x 64
-// room, 8 bounces: 0.41 -> 0.33 ms; 1280 x 720 preview, whose last bounces and
-// tail hold some 1,000 paths: 1.44 -> 1.22 ms.
-constexpr uint32_t kCoopMax = 148u * 32u * 4u;
+// Launched after k_extend / k_shadow where the queue may be short (forms); its
+// length decides on the device which of the two does the work (kCoopMax).
+// 64 x 64 room, 8 bounces: 0.41 -> 0.33 ms; 1280 x 720 preview, whose last
+// bounces and tail hold some 1,000 paths: 1.44 -> 1.22 ms.
 constexpr int kCoopBlock = 64;
 constexpr uint32_t kCoopTailMax = kCoopMax / 4;  // k_tail8: 8 blocks of 64 per SM (128 registers)
 __device__ __forceinline__ uint32_t claim4(uint32_t *next) {
@@ -1603,9 +1601,10 @@ __global__ void __launch_bounds__(kBlock, ShadeBlocks<CLS>::value) k_shade(const
 // kernels still last as long as their slowest ray (about 0.23 ms per bounce
 // of the bench frame, 12 bounces of 16).  When at most kTailMaxPaths paths
 // are left, k_tail runs each to its end in one thread, its next ray kept in
-// the path's own queue position, and k_tail_close empties the queue so the
-// per-bounce kernels that follow (launched either way) find nothing; with
-// more paths left k_tail returns at once and the per-bounce kernels go on.
+// the path's own queue position (k_tail8, for at most kCoopTailMax paths: in 8
+// lanes that share its traversals), and k_tail_close empties the queue: the
+// per-bounce kernels that follow are the body of a conditional graph node and
+// do not run.  With more paths left k_tail returns at once and they go on.
 // It is launched only when at least kTailMinRemaining bounces remain: one
 // thread per path keeps a warp's finished lanes idle until its longest path
 // ends (the per-bounce kernels compact them away every bounce), so the tail
@@ -2011,10 +2010,11 @@ int counters_alloc(pt_ctx *ctx, uint32_t depth) {
 // results that only the next shading pass reads), so in a graph they are
 // parallel nodes: with few paths each kernel lasts as long as its slowest
 // thread, and a bounce then costs two such times instead of one per kernel.
-// Measured, one stream -> branches (with one memset per wave instead of three
-// per bounce, the conditional body and the launch shapes below): 64 x 64 room
-// 0.75 -> 0.40 ms, 1280 x 720 preview 1.91 -> 1.41 ms, fog scene at 1917 x
-// 1079 x 4 17.4 -> 15.5 ms, 59 M-path frame 27.2 -> 26.9 ms.
+// Measured, one stream -> six branches (with one memset per wave instead of
+// three per bounce, the conditional body and the launch shapes below): 64 x 64
+// room 0.75 -> 0.40 ms, 1280 x 720 preview 1.91 -> 1.41 ms, fog scene at 1917 x
+// 1079 x 4 17.4 -> 15.5 ms, 59 M-path frame 27.2 -> 26.9 ms.  One branch
+// (kBranches) keeps these within 0.01 ms.
 struct ForkJoin {
     const cudaStream_t *branch;
     cudaEvent_t forkEv;
